@@ -35,7 +35,8 @@ enum BufId {
   B_ROWKEYS, B_DONE_ROW, B_WORK, B_WFA_MAXS, B_WFA_TBF, B_WFA_OUT, B_WFA_NCIG, B_WFA_SLOTS,
   B_WFA_SCRATCH, B_WFA_FLAGS, B_PF_CHAINS, B_PF_TOP1, B_PF_MARGIN, B_PF_OUT, B_PF_NCIG,
   B_PF_MDLEN, B_PF_MDOFF, B_PF_MD, B_PF_EXACT, B_WFA_FB, B_WFA_WHIST, B_SIEVE_LIST, B_PACKED, B_STATUS, B_KEEP, B_ROW_OFF,
-  B_ROWS, B_ROW_SUMS, B_ROW_TOTAL, B_SW_GROUPS, B_COUNT
+  B_ROWS, B_ROW_SUMS, B_ROW_TOTAL, B_SW_GROUPS, B_RESCUE_LIST, B_RESCUE_TRACE, B_RESCUE_META,
+  B_COUNT
 };
 
 struct DevBuf {
@@ -276,7 +277,7 @@ int plain_shape(uint32_t max_band) {
 }
 
 bool shape_fits(int s, uint32_t max_band) {
-  return s >= 0 && s < kNumBswShapes &&
+  return s >= 0 && s < kNumAllBswShapes &&
          shape_cap(kBswShapes[s]) >= 2 * (int)std::max<uint32_t>(max_band, 1) + 1;
 }
 
@@ -287,10 +288,30 @@ bool shape_usable(int s, uint32_t max_band, uint32_t max_q, const SwParams& sp) 
   return !kBswShapes[s].packed || packed_fits(kBswShapes[s], max_q, sp);
 }
 
-// Default: the first packed shape that covers the band and fits int16, else the
-// int32 shape of the one-launch path.
-int default_shape(uint32_t max_band, uint32_t max_q, const SwParams& sp) {
-  for (int s = 0; s < kNumBswShapes; ++s)
+// Default: the first of kPicks, in the order of their row capacity, that covers the
+// band, has the items to fill the GPU and whose values fit int16. Fewer lanes per pair do
+// less work per cell (a row's scalar work is done once per pair, one lane needs no
+// exchange), more lanes finish a row sooner. Measured DP times at 150 bp, band 33 (1 x 34
+// words, 4 x 9, 8 x 5, 32 x 2): 100,000 items 0.79 / 1.18 / 1.73 / 4.34 ms; 20,000 items
+// 0.29 / 0.29 / 0.37 / 0.90; 8,000 items 0.23 / 0.17 / 0.18 / 0.37; 2,000 items 0.21 /
+// 0.15 / 0.10 / 0.12; 16 items 0.17 / 0.14 / 0.10 / 0.06. Batches no pick fits take any
+// packed shape that does, else the int32 shape of the one-launch path.
+int default_shape(uint32_t max_band, uint32_t max_q, const SwParams& sp, uint32_t items) {
+  struct Pick {
+    int shape;
+    uint32_t min_items;
+  };
+  constexpr Pick kPicks[] = {
+      {23, 20000}, {8, 8000},                // 34 cells on 1 lane, 40 on 4
+      {22, 20000}, {9, 8000},   {10, 1200},  // 68 on 1, 72 on 4, 80 on 8
+      {24, 0},                               // 128 on 32
+      {19, 20000}, {11, 1200},               // 136 on 2, 144 on 8
+      {20, 10000}, {12, 1200},               // 272 on 4, 288 on 16
+      {25, 0},     {13, 0},                  // 320 and 576 on 32
+  };
+  for (const Pick& p : kPicks)
+    if (items >= p.min_items && shape_usable(p.shape, max_band, max_q, sp)) return p.shape;
+  for (int s = 0; s < kNumAllBswShapes; ++s)
     if (kBswShapes[s].packed && shape_usable(s, max_band, max_q, sp)) return s;
   return plain_shape(max_band);
 }
@@ -440,10 +461,18 @@ int build_planes(kira_ctx* ctx, DevPairs& D, uint64_t read_bytes, uint64_t win_b
 
 // Launch shape of the banded SW stage: the tuned choice for the band class if it
 // covers the band, else the smallest shape that does.
-int pick_shape(const kira_ctx* ctx, uint32_t max_band, uint32_t max_q, const SwParams& sp) {
+// (`items`: the items the stage is expected to run).
+int pick_shape(const kira_ctx* ctx, uint32_t max_band, uint32_t max_q, const SwParams& sp,
+               uint32_t items) {
   const int t = ctx->tuned_shape[band_class(max_band)];
-  return shape_usable(t, max_band, max_q, sp) ? t : default_shape(max_band, max_q, sp);
+  return shape_usable(t, max_band, max_q, sp) ? t : default_shape(max_band, max_q, sp, items);
 }
+
+// Items the composed path's banded-SW stage is expected to run for n pairs (the count is
+// only known on the device): most candidates are rejected or certified -- 5 % of the
+// pairs reach it with 8 candidates per read, 10 % with 4, 25 % under the router's own
+// bounds.
+inline uint32_t expected_sw_items(uint32_t n) { return n / 8; }
 
 // Bytes the banded-SW trace arena (trace slots + row metadata) may take: the
 // context's override, else half of the free device memory plus what the arena
@@ -500,6 +529,26 @@ int prepare_bsw(kira_ctx* ctx, uint32_t n_pairs, uint32_t items, uint32_t trace_
   return KIRA_OK;
 }
 
+// Rescue list and trace slots of a banded-SW stage whose packed traces can wrap (`any`:
+// it has a packed shape); `count` is the list's count word, reset with the stage's
+// counters.
+constexpr uint32_t kRescueSlots = 8;
+int prepare_rescue(kira_ctx* ctx, uint32_t items, uint32_t max_q, bool any, const SwParams& sp,
+                   uint32_t* count, BswLaunch& B) {
+  if (!any || !packed_trace_wraps(max_q, sp)) return KIRA_OK;
+  cudaError_t cerr = cudaSuccess;
+  B.rescue_slots = std::min(kRescueSlots, std::max<uint32_t>(items, 1));
+  B.rescue_slot_bytes = (max_q + 1ull) * kRescueRowBytes;
+  KIRA_DBUF(list, uint32_t, B_RESCUE_LIST, std::max<uint32_t>(items, 1));
+  KIRA_DBUF(trace, uint8_t, B_RESCUE_TRACE, B.rescue_slot_bytes * B.rescue_slots);
+  KIRA_DBUF(meta, uint32_t, B_RESCUE_META, (max_q + 1ull) * B.rescue_slots);
+  B.rescue_list = list;
+  B.rescue_count = count;
+  B.rescue_trace = trace;
+  B.rescue_meta = meta;
+  return KIRA_OK;
+}
+
 // DP + traceback of `items` items in rounds of `per_round` (trace slots reused);
 // `between` (profiling) is recorded after the first round's DP.
 // With `work` (dynamic fetch) round r takes its items through counter work[r].
@@ -515,6 +564,11 @@ cudaError_t launch_bsw_rounds(int shape, const DevPairs& D, BswLaunch B, uint32_
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
+}
+
+// After every traceback of a stage: the items whose packed walk was lost, if any can be.
+cudaError_t finish_rescue(const DevPairs& D, const BswLaunch& B, cudaStream_t st) {
+  return B.rescue_list ? launch_bsw_rescue(D, B, st) : cudaSuccess;
 }
 
 // CIGAR scan + compaction over all pairs; writes the total op count to total_dev.
@@ -575,7 +629,7 @@ int verify_pipeline(kira_ctx* ctx, DevPairs D, const Maxes& mx, const kira_verif
   if (rc) return rc;
   if (mx.q > 512) return fail(ctx, KIRA_ERR_READ_TOO_LONG, "read of %u bases > 512", mx.q);
   const SwParams sp = resolve(p.sw);
-  const int shape = pick_shape(ctx, mx.band, mx.q, sp);
+  const int shape = pick_shape(ctx, mx.band, mx.q, sp, expected_sw_items(n));
   if (shape < 0) return fail(ctx, KIRA_ERR_INVALID, "no banded-SW shape for band %u", mx.band);
   uint32_t* ncig = df ? df->ncig + df->base : nullptr;
   int32_t* swoff = df ? df->swoff + df->base : nullptr;
@@ -641,6 +695,8 @@ int verify_pipeline(kira_ctx* ctx, DevPairs D, const Maxes& mx, const kira_verif
   B.out = out;
   B.ncig = ncig;
   B.flags = counters + 2;
+  rc = prepare_rescue(ctx, n, mx.q, kBswShapes[shape].packed, sp, counters + 3, B);
+  if (rc) return rc;
   if (per_round >= n && n >= kSplitPairs && !ctx->profile) {
     // One trace round: the two halves of the banded-SW items (split on the device
     // by the Myers stage's count) run on two streams, so one half's DP fills the
@@ -661,6 +717,7 @@ int verify_pipeline(kira_ctx* ctx, DevPairs D, const Maxes& mx, const kira_verif
     KIRA_CUDA(launch_bsw_rounds(shape, D, B, n, per_round, ctx->sms, st,
                                 ctx->profile ? ctx->ev[3] : nullptr));
   }
+  KIRA_CUDA(finish_rescue(D, B, st));
   if (ctx->profile) ctx->ev_recorded = 4;
   mark(ctx, 4, st);
   if (cm.before_scan) KIRA_CUDA(cudaStreamWaitEvent(st, cm.before_scan, 0));
@@ -682,6 +739,7 @@ struct BucketRun {
   uint32_t one_round, nwork;
   uint32_t* work;
   BswLaunch L[kBandClasses];
+  BswLaunch all;  // the whole batch's list and slots, for the rescue
 };
 
 // Enqueues the launches of a planned bucketed call on `st` (capturable).
@@ -713,7 +771,7 @@ cudaError_t enqueue_bucketed(kira_ctx* ctx, const DevPairs& D, const BucketRun& 
       if (!first && (e = cudaStreamWaitEvent(st, ctx->ev_cls_join[c], 0)) != cudaSuccess) return e;
       first = false;
     }
-    return cudaSuccess;
+    return finish_rescue(D, R.all, st);
   }
   if (R.one_round) {
     // Widest class first (longest rows), then the narrower ones fill in behind it.
@@ -733,6 +791,7 @@ cudaError_t enqueue_bucketed(kira_ctx* ctx, const DevPairs& D, const BucketRun& 
         return e;
     mark(ctx, 3, st);
   }
+  if ((e = finish_rescue(D, R.all, st)) != cudaSuccess) return e;
   mark(ctx, 4, st);
   return cudaSuccess;
 }
@@ -816,7 +875,7 @@ int plan_bucketed(kira_ctx* ctx, const kira_pairs& P, const DevPairs& D, const k
   uint64_t slot[kBandClasses] = {}, per[kBandClasses] = {};
   uint64_t total = 0;
   for (int c = 0; c < kBandClasses; ++c) {
-    shape[c] = cnt[c] ? pick_shape(ctx, bmax[c], qmax[c], sp) : -1;
+    shape[c] = cnt[c] ? pick_shape(ctx, bmax[c], qmax[c], sp, cnt[c]) : -1;
     if (cnt[c] && shape[c] < 0) return fail(ctx, KIRA_ERR_INVALID, "no shape for band %u", bmax[c]);
     if (!cnt[c]) continue;
     slot[c] = trace_slot_bytes(shape[c], qmax[c]);
@@ -880,6 +939,20 @@ int plan_bucketed(kira_ctx* ctx, const kira_pairs& P, const DevPairs& D, const k
   R.one_round = one_round ? 1u : 0u;
   R.nwork = nwork;
   R.work = work;
+  bool packed = false;
+  for (int c = 0; c < kBandClasses; ++c) packed |= cnt[c] && kBswShapes[shape[c]].packed;
+  R.all.list = dlist;
+  R.all.count = n;
+  R.all.sp = sp;
+  R.all.offset = D.band_offset;
+  R.all.cig_slots = slots;
+  R.all.slot_cap = cap;
+  R.all.out = dout;
+  R.all.ncig = ncig;
+  R.all.item_of_pair = iop;
+  R.all.flags = flags_dev;
+  R.all.max_q = qall;
+  if (int rc = prepare_rescue(ctx, n, qall, packed, sp, flags_dev + 1, R.all)) return rc;
   for (int c = 0; c < kBandClasses; ++c) {
     R.shape[c] = shape[c];
     R.cnt[c] = cnt[c];
@@ -904,6 +977,7 @@ int plan_bucketed(kira_ctx* ctx, const kira_pairs& P, const DevPairs& D, const k
     B.max_q = qmax[c];
     B.work = work + rounds_before[c];
     B.item_base = base[c];
+    if (sh.packed) B.rescue_list = R.all.rescue_list, B.rescue_count = R.all.rescue_count;
   }
   G = BswLaunch{};
   G.item_of_pair = iop;
@@ -1232,9 +1306,9 @@ int verify_batch_chunked(kira_ctx* ctx, const kira_pairs& P, const kira_verify_p
       gm.w = std::max(gm.w, scans[c].mx.w);
       gm.band = std::max(gm.band, scans[c].mx.band);
     }
-    const int shape = pick_shape(ctx, gm.band, gm.q, gsp);
-    if (shape < 0) return fail(ctx, KIRA_ERR_INVALID, "no banded-SW shape for band %u", gm.band);
     const uint32_t lo = bounds[c0], ng = bounds[c1] - lo;
+    const int shape = pick_shape(ctx, gm.band, gm.q, gsp, expected_sw_items(ng));
+    if (shape < 0) return fail(ctx, KIRA_ERR_INVALID, "no banded-SW shape for band %u", gm.band);
     const uint32_t per_round = round_items(gx, ng, shape, gm.q);
     BswLaunch& B = gB[g];
     int rc = prepare_bsw(gx, n, ng, per_round, gm, shape, B);
@@ -1251,6 +1325,11 @@ int verify_batch_chunked(kira_ctx* ctx, const kira_pairs& P, const kira_verify_p
     B.out = dout;
     B.ncig = dfs.ncig;
     B.flags = static_cast<uint32_t*>(gx->bufs[B_COUNTERS].p) + 2;
+    rc = prepare_rescue(gx, ng, gm.q, kBswShapes[shape].packed, gsp, B.flags + 1, B);
+    if (rc) {
+      if (gx != ctx) ctx->last_error = gx->last_error;
+      return rc;
+    }
     // The group's scratch was (re)sized on gx's stream; its chunks' fronts ran on
     // both compute streams.
     KIRA_CUDA(cudaEventRecord(ctx->ev_cls_join[2 + g], gx->stream));
@@ -1270,6 +1349,7 @@ int verify_batch_chunked(kira_ctx* ctx, const kira_pairs& P, const kira_verify_p
     } else {
       KIRA_CUDA(launch_bsw_rounds(shape, Dg, B, ng, per_round, ctx->sms, s1, nullptr));
     }
+    KIRA_CUDA(finish_rescue(Dg, B, s1));
     KIRA_CUDA(cudaEventRecord(ctx->ev_cls_join[g], s1));
     return KIRA_OK;
   };
@@ -1872,7 +1952,7 @@ int kira_gpu_sieve_batch(kira_ctx* ctx, const kira_sieve_job* jobs, uint32_t n,
 
 int kira_gpu_set_bsw_shape(kira_ctx* ctx, uint32_t band, int shape) {
   if (!ctx) return KIRA_ERR_INVALID;
-  if (shape >= 0 && !shape_fits(shape, band))
+  if (shape >= 0 && (shape >= kNumBswShapes || !shape_fits(shape, band)))
     return fail(ctx, KIRA_ERR_INVALID, "shape %d does not cover band %u", shape, band);
   ctx->tuned_shape[band_class(band)] = shape;
   return KIRA_OK;
@@ -2663,7 +2743,7 @@ int kira_gpu_bsw_batch(kira_ctx* ctx, const kira_pairs* pairs, const kira_sw_cfg
     // packed int16 wherever the scores fit, else int32), one launch over every pair
     // in input order; only the bucketing, dynamic fetch and graph replay differ.
     const SwParams sp = resolve(*cfg);
-    const int shape = pick_shape(ctx, mx.band, mx.q, sp);
+    const int shape = pick_shape(ctx, mx.band, mx.q, sp, n);
     if (shape < 0)
       return fail(ctx, KIRA_ERR_INVALID, "band %u above the one-launch maximum", mx.band);
     const uint32_t per_round = round_items(ctx, n, shape, mx.q);
@@ -2678,9 +2758,12 @@ int kira_gpu_bsw_batch(kira_ctx* ctx, const kira_pairs* pairs, const kira_sw_cfg
     B.out = dout;
     B.ncig = ncig;
     B.flags = counters + 2;
+    rc = prepare_rescue(ctx, n, mx.q, kBswShapes[shape].packed, sp, counters + 3, B);
+    if (rc) return rc;
     mark(ctx, 2, st);
     KIRA_CUDA(launch_bsw_rounds(shape, D, B, n, per_round, ctx->sms, st,
                                 ctx->profile ? ctx->ev[3] : nullptr));
+    KIRA_CUDA(finish_rescue(D, B, st));
     if (ctx->profile) ctx->ev_recorded = 4;
     mark(ctx, 4, st);
     rc = finish_cigars(ctx, n, dout, ncig, B, ops, cigar->cap, total_dev, st);

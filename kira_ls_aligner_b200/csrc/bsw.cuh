@@ -328,19 +328,21 @@ __device__ __forceinline__ uint32_t warp_walk(const Code& code, int32_t& i, int3
 }
 
 // Trace codes of the int32 sweep of shape <G, K>: one nibble per cell, already in
-// warp_walk's code layout; lane gi of the row holds band cells gi*K .. +K-1.
-template <int G, int K>
+// warp_walk's code layout; lane gi of the row holds band cells gi*K .. +K-1. FRESH:
+// the same kernel wrote the trace (no read-only loads).
+template <int G, int K, bool FRESH = false>
 struct BswCode {
   const uint8_t* __restrict__ trace;
   const uint32_t* __restrict__ meta;
   __device__ __forceinline__ uint32_t operator()(int32_t i, int32_t j) const {
     constexpr uint32_t LB = BswShape<G, K>::kLaneBytes, S = BswShape<G, K>::kRowStride;
-    const uint32_t m = __ldg(meta + i);
+    const uint32_t m = FRESH ? *const_cast<const volatile uint32_t*>(meta + i) : __ldg(meta + i);
     const int32_t rs = (int32_t)(m >> 11), rl = (int32_t)(m & 2047u);
     const int32_t idx = j - rs;
     if (idx < 0 || idx >= rl) return 0xFFu;
     const uint32_t gi = (uint32_t)idx / (uint32_t)K, kk = (uint32_t)idx - gi * (uint32_t)K;
-    const uint32_t byte = __ldg(trace + (size_t)i * S + gi * LB + (kk >> 1));
+    const uint8_t* at = trace + (size_t)i * S + gi * LB + (kk >> 1);
+    const uint32_t byte = FRESH ? *const_cast<const volatile uint8_t*>(at) : __ldg(at);
     return (byte >> ((kk & 1u) * 4u)) & 15u;
   }
 };

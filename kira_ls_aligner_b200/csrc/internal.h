@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace kira {
@@ -97,6 +99,16 @@ struct BswLaunch {
   // 1 / 2: the first / second half of the item count (device-side), for the two
   // halves of a one-round batch run on two streams at once; 0: the round above.
   uint32_t split;
+  // Packed shapes on batches whose scores pass 255 (the trace keeps H mod 256): items
+  // whose walk ended with a value left over (warp_walk_h) are listed here as item_base
+  // + item, and bsw_rescue_kernel aligns them again on int32 lanes, `rescue_slots` at
+  // a time over its own trace slots. Null: no walk can lose its value.
+  uint32_t* rescue_list;
+  uint32_t* rescue_count;
+  uint8_t* rescue_trace;
+  uint32_t* rescue_meta;      // max_q + 1 words per slot
+  uint64_t rescue_slot_bytes;
+  uint32_t rescue_slots;
 };
 
 struct CompactLaunch {
@@ -205,13 +217,14 @@ struct BswShapeInfo {
   int g, k, threads, min_blocks, packed;
 };
 extern const BswShapeInfo kBswShapes[];
-extern const int kNumBswShapes;
+extern const int kNumBswShapes;     // the listed shapes (kira_gpu_bsw_shapes)
+extern const int kNumAllBswShapes;  // and the ones only the default pick uses, after them
 
 inline int shape_cap(const BswShapeInfo& s) { return (s.packed ? 2 : 1) * s.g * s.k; }
 inline uint32_t shape_lane_bytes(const BswShapeInfo& s) {
-  // packed: a 4-bit code per cell, four words (eight cells) per 4-byte slab;
+  // packed: a byte per cell, two words (four cells) per 4-byte slab;
   // int32: a 4-bit code per cell, eight cells per 4 bytes.
-  return s.packed ? 4u * (uint32_t)((s.k + 3) / 4) : 4u * (uint32_t)((s.k + 7) / 8);
+  return s.packed ? 4u * (uint32_t)((s.k + 1) / 2) : 4u * (uint32_t)((s.k + 7) / 8);
 }
 inline uint32_t shape_row_stride(const BswShapeInfo& s) {
   return (uint32_t)s.g * shape_lane_bytes(s);
@@ -219,7 +232,7 @@ inline uint32_t shape_row_stride(const BswShapeInfo& s) {
 // Rows per interleave block of the packed trace (Bsw16Shape::kInterleave).
 inline uint32_t shape_row_interleave(const BswShapeInfo& s) {
   if (!s.packed) return 1u;
-  return s.g == 1 ? 8u : s.g < 32 ? 32u / (uint32_t)s.g : 1u;
+  return s.g <= 4 ? 8u : s.g < 32 ? 32u / (uint32_t)s.g : 1u;
 }
 // Bytes of one item's trace slot for reads of up to `max_q` bases: rows 0..max_q
 // rounded up to whole interleave blocks, then to 16 bytes.
@@ -245,15 +258,13 @@ inline int packed_key_bits(int k) {
   return k <= 2 ? 1 : k <= 4 ? 2 : k <= 8 ? 3 : k <= 16 ? 4 : k <= 32 ? 5 : 6;
 }
 
-// The packed sweep is exact when every biased value stays below 2^13, every
-// difference its flags test stays below 2^11 (the F-extend flag at bit 11), and
-// every biased H fits a row-max key (H << key bits below 2^16).
+// The packed sweep is exact when every biased value stays below 2^13 and every biased H
+// fits a row-max key (H << key bits below 2^16).
 inline bool packed_fits(const BswShapeInfo& s, uint32_t max_q, const SwParams& sp) {
   if (!s.packed) return false;
   if (sp.match < 0 || sp.mismatch < 0 || sp.gap_open < 0 || sp.gap_extend < 0) return false;
   const int64_t top = (int64_t)max_q * sp.match;
   const int64_t cap = shape_cap(s);
-  if (top + cap * sp.gap_extend + sp.gof >= 2048) return false;
   if (top + (int64_t)packed_bias(s, sp) >= (int64_t(1) << (16 - packed_key_bits(s.k))))
     return false;
   return top + (int64_t)packed_bias(s, sp) + cap * sp.gap_extend < 8192;
@@ -287,6 +298,18 @@ constexpr int kBswPartDp = 1, kBswPartTb = 2;
 cudaError_t launch_bsw(int shape, const DevPairs& P, const BswLaunch& B, uint32_t max_items,
                        int sms, cudaStream_t st, cudaEvent_t between = nullptr,
                        int parts = kBswPartDp | kBswPartTb);
+// Aligns the items the packed tracebacks listed in B.rescue_list again (B: the whole
+// batch's list, ends and CIGAR slots); nothing to do on nearly every batch.
+cudaError_t launch_bsw_rescue(const DevPairs& P, const BswLaunch& B, cudaStream_t st);
+// Trace row of the rescue's int32 sweep (576 cells, the widest listed row).
+constexpr int kRescueLanes = 32, kRescueCells = 18;
+constexpr uint64_t kRescueRowBytes = 4ull * kRescueLanes * ((kRescueCells + 7) / 8);
+// The packed trace keeps H mod 256. A walk's comparisons are between values of at most
+// max_q * match and differ from them by a mismatch or one gap step: it can lose its
+// value only when those pass 255.
+inline bool packed_trace_wraps(uint32_t max_q, const SwParams& sp) {
+  return (int64_t)max_q * sp.match + std::max(sp.mismatch, sp.gof + sp.gap_extend) > 255;
+}
 cudaError_t launch_cigar_scan(const uint32_t* ncig, uint32_t n, uint32_t* off,
                               uint32_t* chunk_sums, uint64_t* total_dev, cudaStream_t st,
                               bool accumulate = false);

@@ -574,11 +574,11 @@ __global__ void __launch_bounds__(T, MINB) bsw_dp_kernel(DevPairs P, BswLaunch B
 // Packed int16 sweep (bsw16.cuh); same item loop and outputs as bsw_dp_kernel.
 template <int G, int K, int T, int MINB>
 __global__ void __launch_bounds__(T, MINB) bsw16_dp_kernel(DevPairs P, BswLaunch B) {
-  // Dynamic shared memory: each group's trace strip (one interleave block,
-  // kStripBytes), then each group's realignment buffer (4 * G * K halves).
+  // Dynamic shared memory: each group's trace strip (one interleave block; groups of
+  // fewer than 8 lanes), then each group's realignment buffer (short lanes).
   extern __shared__ __align__(128) uint32_t bsw16_smem[];
   constexpr int CAP = 2 * G * K;
-  constexpr uint32_t kStripWords = Bsw16Shape<G, K>::kStripBytes / 4u;
+  constexpr uint32_t kStripWords = Bsw16Shape<G, K>::kStripStride / 4u;
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t g = lane % G;
   const uint32_t gw = lane / G;
@@ -587,7 +587,7 @@ __global__ void __launch_bounds__(T, MINB) bsw16_dp_kernel(DevPairs P, BswLaunch
   const uint32_t group_in_block = threadIdx.x / G;
   uint32_t* strip = bsw16_smem + (size_t)group_in_block * kStripWords;
   uint16_t* rowbuf = reinterpret_cast<uint16_t*>(bsw16_smem + (size_t)(T / G) * kStripWords) +
-                     (size_t)group_in_block * 4u * G * K;  // per group
+                     (size_t)group_in_block * (Bsw16Shape<G, K>::kRowBytes / 2);
   uint32_t lo, count;
   bsw_range(B, lo, count);
   const uint32_t ngroups = gridDim.x * groups_per_block;
@@ -628,8 +628,29 @@ __global__ void __launch_bounds__(T, MINB) bsw16_dp_kernel(DevPairs P, BswLaunch
   if (g == 0) bulk_copies_done();  // the trace copies this lane issued
 }
 
-// One warp per item (warp_walk over the trace of shape <G, K>, packed or int32);
-// lane 0 writes the item's result row.
+// An item's result row, from its end and where its walk stopped (i, j).
+__device__ __forceinline__ void write_sw_row(const BswLaunch& B, uint32_t item, uint32_t pair,
+                                             const DpEnd& e, bool outside, int32_t i, int32_t j,
+                                             uint32_t n, uint32_t overflow) {
+  kira_sw_result r;
+  r.score = e.score;
+  r.ref_start = (uint32_t)j;
+  r.ref_end = (uint32_t)e.end_j;
+  r.read_start = i;
+  r.read_end = e.end_i;
+  r.cigar_off = 0;
+  r.n_cigar = n;
+  r.status = outside ? KIRA_PAIR_OUT_OF_BOUNDS : KIRA_PAIR_SW;
+  r.early_abort = outside ? 0 : (uint8_t)e.early_abort;
+  r.reserved = overflow ? 1 : 0;
+  B.out[pair] = r;
+  B.ncig[pair] = n;
+  B.item_of_pair[pair] = B.item_base + item;
+  if (overflow) atomicOr(B.flags, 1u);
+}
+
+// One warp per item (the walk over the trace of shape <G, K>: warp_walk_h packed,
+// warp_walk int32); lane 0 writes the item's result row.
 constexpr uint32_t kTbStageBytes = 4096;  // per warp: metadata + read + window of a walk
 
 template <int G, int K, bool PACKED>
@@ -650,6 +671,7 @@ __global__ void __launch_bounds__(128) bsw_tb_kernel(DevPairs P, BswLaunch B) {
     const uint32_t* mt = B.tg.meta + (size_t)slot_item * B.tg.meta_stride;
     uint32_t* ops = B.cig_slots + (size_t)item * B.slot_cap;
     uint32_t n = 0;
+    bool lost = false;
     const bool outside = e.early_abort == kEndOutsideShape;  // uniform over the warp
     if (outside) {
       i = j = 0;
@@ -660,6 +682,7 @@ __global__ void __launch_bounds__(128) bsw_tb_kernel(DevPairs P, BswLaunch B) {
       const uint32_t q = P.read_len[pair], w = P.win_len[pair];
       const uint8_t* rd = P.read_seq + P.read_off[pair];
       const uint8_t* wn = P.win_seq + P.win_off[pair];
+      const uint32_t zero = (uint32_t)(B.bias - B.sp.gof);  // the stored H = 0
       if (4u * (q + 1u) + q + w <= kTbStageBytes) {
         uint32_t* smeta = tb_stage[threadIdx.x >> 5];
         uint8_t* sseq = reinterpret_cast<uint8_t*>(smeta + q + 1u);
@@ -668,32 +691,53 @@ __global__ void __launch_bounds__(128) bsw_tb_kernel(DevPairs P, BswLaunch B) {
         for (uint32_t t = ln; t < q; t += 32u) sseq[t] = __ldg(rd + t);
         for (uint32_t t = ln; t < w; t += 32u) sseq[q + t] = __ldg(wn + t);
         __syncwarp();
-        n = warp_walk_scored(Bsw16Code<G, K, true>{tr, smeta, B.sp.gap_open}, i, j, e.score,
-                             sseq, sseq + q, B.sp, ops, B.slot_cap, overflow);
+        n = warp_walk_h(Bsw16Trace<G, K, true>{tr, smeta, zero}, i, j, e.score, sseq, sseq + q,
+                        B.sp, ops, B.slot_cap, overflow, lost);
         __syncwarp();
       } else {
-        n = warp_walk_scored(Bsw16Code<G, K>{tr, mt, B.sp.gap_open}, i, j, e.score, rd, wn,
-                             B.sp, ops, B.slot_cap, overflow);
+        n = warp_walk_h(Bsw16Trace<G, K>{tr, mt, zero}, i, j, e.score, rd, wn, B.sp, ops,
+                        B.slot_cap, overflow, lost);
       }
     } else {
       n = warp_walk(BswCode<G, K>{tr, mt}, i, j, ops, B.slot_cap, overflow);
     }
     if (!lead) continue;
-    kira_sw_result r;
-    r.score = e.score;
-    r.ref_start = (uint32_t)j;
-    r.ref_end = (uint32_t)e.end_j;
-    r.read_start = i;
-    r.read_end = e.end_i;
-    r.cigar_off = 0;
-    r.n_cigar = n;
-    r.status = outside ? KIRA_PAIR_OUT_OF_BOUNDS : KIRA_PAIR_SW;
-    r.early_abort = outside ? 0 : (uint8_t)e.early_abort;
-    r.reserved = overflow ? 1 : 0;
-    B.out[pair] = r;
-    B.ncig[pair] = n;
-    B.item_of_pair[pair] = B.item_base + item;
-    if (overflow) atomicOr(B.flags, 1u);
+    if (lost) {
+      if (B.rescue_list) B.rescue_list[atomicAdd(B.rescue_count, 1u)] = B.item_base + item;
+      else atomicOr(B.flags, 1u);
+      continue;
+    }
+    write_sw_row(B, item, pair, e, outside, i, j, n, overflow);
+  }
+}
+
+// Items whose packed walk lost its value: the int32 sweep and its walk, one warp (and
+// one trace slot) per item. Runs after every traceback of the batch.
+__global__ void __launch_bounds__(32) bsw_rescue_kernel(DevPairs P, BswLaunch B) {
+  constexpr int G = kRescueLanes, K = kRescueCells;
+  __shared__ int32_t rowbuf[2 * K * 32];
+  const uint32_t count = *B.rescue_count;
+  uint8_t* tr = B.rescue_trace + (size_t)blockIdx.x * B.rescue_slot_bytes;
+  uint32_t* mt = B.rescue_meta + (size_t)blockIdx.x * (B.max_q + 1u);
+  for (uint32_t e = blockIdx.x; e < count; e += gridDim.x) {
+    const uint32_t item = B.rescue_list[e];
+    const uint32_t pair = B.list ? B.list[item] : item;
+    const int32_t band = max(P.bandwidth ? P.bandwidth[pair] : B.sp.band, 1);
+    DpEnd end;
+    uint64_t cells = 0;
+    bsw_group_sweep<G, K, false>(P.read_seq + P.read_off[pair], P.read_len[pair],
+                                 P.win_seq + P.win_off[pair], P.win_len[pair], band,
+                                 B.offset ? B.offset[pair] : 0,
+                                 P.abort_score ? P.abort_score[pair] : kAbortOff, B.sp, rowbuf, 0u,
+                                 tr, mt, threadIdx.x, 0xFFFFFFFFu, end, cells, nullptr);
+    __threadfence_block();
+    __syncwarp();
+    int32_t i = end.end_i, j = end.end_j;
+    uint32_t overflow = 0;
+    const uint32_t n = warp_walk(BswCode<G, K, true>{tr, mt}, i, j,
+                                 B.cig_slots + (size_t)item * B.slot_cap, B.slot_cap, overflow);
+    if (threadIdx.x == 0) write_sw_row(B, item, pair, end, false, i, j, n, overflow);
+    __syncwarp();
   }
 }
 
@@ -995,8 +1039,8 @@ static cudaError_t launch_bsw16_shape(const DevPairs& P, const BswLaunch& B, uin
                                       int sms, cudaStream_t st, cudaEvent_t between, int parts) {
   cudaError_t e = cudaSuccess;
   if (parts & kBswPartDp) {
-    // per group: a trace strip of kStripBytes and 4 * G * K halves
-    const size_t smem = (size_t)(T / G) * Bsw16Shape<G, K>::kStripBytes + (size_t)T * 8u * K;
+    const size_t smem =
+        (size_t)(T / G) * (Bsw16Shape<G, K>::kStripStride + Bsw16Shape<G, K>::kRowBytes);
     auto kern = bsw16_dp_kernel<G, K, T, MINB>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int per_sm = 0;
@@ -1017,54 +1061,59 @@ static cudaError_t launch_bsw16_shape(const DevPairs& P, const BswLaunch& B, uin
 }
 
 // Launch shapes (lanes per pair, cells per lane, threads per block, min resident
-// blocks per SM). The host picks the first shape whose G*K covers 2*band+1
-// unless a tuned choice is installed for the band (autotuner / override).
+// blocks per SM). Installed per band class by the autotuner / override, else picked by
+// default_shape.
 const BswShapeInfo kBswShapes[] = {
     {4, 10, 256, 2, 0},  {4, 17, 128, 4, 0},  {4, 17, 128, 3, 0}, {8, 10, 256, 2, 0},
     {8, 17, 128, 3, 0},  {16, 17, 128, 3, 0}, {32, 17, 128, 3, 0},
-    // packed int16: K words = 2K cells per lane
-    {2, 9, 256, 2, 1},   {4, 5, 256, 2, 1},   {4, 9, 256, 2, 1},  {8, 5, 256, 2, 1},
-    {8, 9, 256, 2, 1},   {16, 9, 256, 2, 1},  {32, 9, 256, 2, 1}, {2, 17, 128, 3, 1},
-    {2, 18, 128, 3, 1},
-    // the same packed sweeps held to more resident blocks (fewer registers, some spilled)
-    {4, 9, 256, 3, 1},   {2, 17, 128, 4, 1},
+    // packed int16: K words = 2K cells per lane. One-warp blocks: a block's SM share
+    // frees up as soon as its own pairs are done.
+    {2, 9, 32, 16, 1},   {4, 5, 32, 16, 1},   {4, 9, 32, 16, 1},  {8, 5, 32, 20, 1},
+    {8, 9, 32, 16, 1},   {16, 9, 32, 16, 1},  {32, 9, 32, 16, 1}, {2, 17, 128, 4, 1},
+    {2, 18, 128, 4, 1},
+    {4, 9, 128, 5, 1},   {2, 17, 32, 16, 1},
     // 34 words a lane: one lane per pair (no cross-lane exchange, a row's scalar
     // work done once), and 2 / 4 lanes for bands up to 67 / 135
-    {1, 34, 128, 2, 1},  {2, 34, 128, 2, 1},  {4, 34, 128, 2, 1},
+    {1, 34, 128, 3, 1},  {2, 34, 128, 3, 1},  {4, 34, 128, 2, 1},
     // one lane per pair in smaller blocks (a block's SMs free up at a finer grain
     // at the end of a launch)
-    {1, 34, 64, 4, 1},   {1, 34, 32, 8, 1},
+    {1, 34, 64, 6, 1},   {1, 34, 32, 12, 1},
+    // ---- not listed (kNumBswShapes): only the default pick uses the shapes below
+    // one lane of 34 cells, for bands up to 16
+    {1, 17, 32, 16, 1},
+    // a warp per pair with the fewest words a lane, for the shortest rows: bands up to
+    // 63 and 159
+    {32, 2, 32, 16, 1},  {32, 5, 32, 16, 1},
 };
-const int kNumBswShapes = sizeof(kBswShapes) / sizeof(kBswShapes[0]);
+const int kNumBswShapes = 23;
+const int kNumAllBswShapes = sizeof(kBswShapes) / sizeof(kBswShapes[0]);
 
 cudaError_t launch_bsw(int shape, const DevPairs& P, const BswLaunch& B, uint32_t max_items,
                        int sms, cudaStream_t st, cudaEvent_t between, int parts) {
   switch (shape) {
-    case 0: return launch_bsw_shape<4, 10, 256, 2>(P, B, max_items, sms, st, between, parts);
-    case 1: return launch_bsw_shape<4, 17, 128, 4>(P, B, max_items, sms, st, between, parts);
-    case 2: return launch_bsw_shape<4, 17, 128, 3>(P, B, max_items, sms, st, between, parts);
-    case 3: return launch_bsw_shape<8, 10, 256, 2>(P, B, max_items, sms, st, between, parts);
-    case 4: return launch_bsw_shape<8, 17, 128, 3>(P, B, max_items, sms, st, between, parts);
-    case 5: return launch_bsw_shape<16, 17, 128, 3>(P, B, max_items, sms, st, between, parts);
-    case 6: return launch_bsw_shape<32, 17, 128, 3>(P, B, max_items, sms, st, between, parts);
-    case 7: return launch_bsw16_shape<2, 9, 256, 2>(P, B, max_items, sms, st, between, parts);
-    case 8: return launch_bsw16_shape<4, 5, 256, 2>(P, B, max_items, sms, st, between, parts);
-    case 9: return launch_bsw16_shape<4, 9, 256, 2>(P, B, max_items, sms, st, between, parts);
-    case 10: return launch_bsw16_shape<8, 5, 256, 2>(P, B, max_items, sms, st, between, parts);
-    case 11: return launch_bsw16_shape<8, 9, 256, 2>(P, B, max_items, sms, st, between, parts);
-    case 12: return launch_bsw16_shape<16, 9, 256, 2>(P, B, max_items, sms, st, between, parts);
-    case 13: return launch_bsw16_shape<32, 9, 256, 2>(P, B, max_items, sms, st, between, parts);
-    case 14: return launch_bsw16_shape<2, 17, 128, 3>(P, B, max_items, sms, st, between, parts);
-    case 15: return launch_bsw16_shape<2, 18, 128, 3>(P, B, max_items, sms, st, between, parts);
-    case 16: return launch_bsw16_shape<4, 9, 256, 3>(P, B, max_items, sms, st, between, parts);
-    case 17: return launch_bsw16_shape<2, 17, 128, 4>(P, B, max_items, sms, st, between, parts);
-    case 18: return launch_bsw16_shape<1, 34, 128, 2>(P, B, max_items, sms, st, between, parts);
-    case 19: return launch_bsw16_shape<2, 34, 128, 2>(P, B, max_items, sms, st, between, parts);
-    case 20: return launch_bsw16_shape<4, 34, 128, 2>(P, B, max_items, sms, st, between, parts);
-    case 21: return launch_bsw16_shape<1, 34, 64, 4>(P, B, max_items, sms, st, between, parts);
-    case 22: return launch_bsw16_shape<1, 34, 32, 8>(P, B, max_items, sms, st, between, parts);
+#define KIRA_BSW(S, G, K, T, M) \
+  case S: return launch_bsw_shape<G, K, T, M>(P, B, max_items, sms, st, between, parts);
+#define KIRA_BSW16(S, G, K, T, M) \
+  case S: return launch_bsw16_shape<G, K, T, M>(P, B, max_items, sms, st, between, parts);
+    KIRA_BSW(0, 4, 10, 256, 2) KIRA_BSW(1, 4, 17, 128, 4) KIRA_BSW(2, 4, 17, 128, 3)
+    KIRA_BSW(3, 8, 10, 256, 2) KIRA_BSW(4, 8, 17, 128, 3) KIRA_BSW(5, 16, 17, 128, 3)
+    KIRA_BSW(6, 32, 17, 128, 3)
+    KIRA_BSW16(7, 2, 9, 32, 16) KIRA_BSW16(8, 4, 5, 32, 16) KIRA_BSW16(9, 4, 9, 32, 16)
+    KIRA_BSW16(10, 8, 5, 32, 20) KIRA_BSW16(11, 8, 9, 32, 16) KIRA_BSW16(12, 16, 9, 32, 16)
+    KIRA_BSW16(13, 32, 9, 32, 16) KIRA_BSW16(14, 2, 17, 128, 4) KIRA_BSW16(15, 2, 18, 128, 4)
+    KIRA_BSW16(16, 4, 9, 128, 5) KIRA_BSW16(17, 2, 17, 32, 16) KIRA_BSW16(18, 1, 34, 128, 3)
+    KIRA_BSW16(19, 2, 34, 128, 3) KIRA_BSW16(20, 4, 34, 128, 2) KIRA_BSW16(21, 1, 34, 64, 6)
+    KIRA_BSW16(22, 1, 34, 32, 12) KIRA_BSW16(23, 1, 17, 32, 16) KIRA_BSW16(24, 32, 2, 32, 16)
+    KIRA_BSW16(25, 32, 5, 32, 16)
+#undef KIRA_BSW
+#undef KIRA_BSW16
     default: return cudaErrorInvalidValue;
   }
+}
+
+cudaError_t launch_bsw_rescue(const DevPairs& P, const BswLaunch& B, cudaStream_t st) {
+  (bsw_rescue_kernel<<<B.rescue_slots, 32, 0, st>>>(P, B), count_launch());
+  return cudaGetLastError();
 }
 
 cudaError_t launch_cigar_scan(const uint32_t* ncig, uint32_t n, uint32_t* off, uint32_t* chunk_sums,
