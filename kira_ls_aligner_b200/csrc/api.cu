@@ -647,7 +647,8 @@ int verify_pipeline(kira_ctx* ctx, DevPairs D, const Maxes& mx, const kira_verif
   KIRA_CUDA(cudaMemsetAsync(counters, 0, cm.first ? 16 : 8, st));
   VerifyDev V{p.sieve_threshold, p.cert_strict, sp,       out,       detail, ncig,
               swoff,             mlist,         counters, p.myers_k, (p.flags & KIRA_VERIFY_NO_QGRAM) ? 0 : 1,
-              nullptr,           nullptr};
+              nullptr,           nullptr,       slist,    df ? df->count : counters + 1,
+              df ? df->base : 0u};
   if (!detail && V.qgram) {  // filter-first sieve: survivor list after its count word
     KIRA_DBUF(sl, uint32_t, B_SIEVE_LIST, (uint64_t)n + 1);
     V.sieve_count = sl;

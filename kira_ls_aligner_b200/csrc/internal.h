@@ -40,6 +40,11 @@ struct VerifyDev {
   // certify; *sieve_count entries. Null: one kernel sieves every pair.
   uint32_t* sieve_list;
   uint32_t* sieve_count;
+  // Filter-first form: pairs whose best shift has at most k mismatches go straight to the
+  // banded-SW list (as sw_base + pair).
+  uint32_t* sw_list;
+  uint32_t* sw_count;
+  uint32_t sw_base;
 };
 
 struct MyersLaunch {

@@ -54,10 +54,11 @@ __global__ void __launch_bounds__(256) sieve_dropin_kernel(SieveJobsDev J,
 // every byte is ((b >> 1) ^ (b >> 2)) & 3 (base_code), a PRMT table lookup gives
 // the letter that code stands for, and the case-folded byte equals it exactly for
 // A, C, G, T. A multiply by 0x01020408 gathers bit 0 of each byte into bits
-// 24..27. The even lane of each pair stores the block of its 32 bases.
+// 24..27 (a fourth nibble marks the valid bytes that are upper case). The even lane of
+// each pair stores the block of its 32 bases.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void plane_nibbles(uint32_t w, uint32_t& n0, uint32_t& n1,
-                                              uint32_t& nv) {
+                                              uint32_t& nv, uint32_t& nu) {
   const uint32_t x = (w >> 1) ^ (w >> 2);       // bits 0-1 of each byte: the code
   const uint32_t y = x & 0x03030303u;
   const uint32_t z = y | (y >> 4);              // bytes 0 and 2: two codes each
@@ -70,6 +71,8 @@ __device__ __forceinline__ void plane_nibbles(uint32_t w, uint32_t& n0, uint32_t
   n0 = ((x & v) * 0x01020408u) >> 24;
   n1 = (((x >> 1) & v) * 0x01020408u) >> 24;
   nv = (v * 0x01020408u) >> 24;
+  // The letter itself: valid and the case bit (0x20) clear.
+  nu = ((v & ~(w >> 5)) * 0x01020408u) >> 24;
 }
 
 __global__ void __launch_bounds__(256) pack_planes_kernel(const uint8_t* __restrict__ seq,
@@ -97,79 +100,28 @@ __global__ void __launch_bounds__(256) pack_planes_kernel(const uint8_t* __restr
         w[k] = x;
       }
     }
-    uint32_t b0 = 0, b1 = 0, bv = 0;
+    uint32_t b0 = 0, b1 = 0, bv = 0, bu = 0;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      uint32_t n0, n1, nv;
-      plane_nibbles(w[k], n0, n1, nv);
+      uint32_t n0, n1, nv, nu;
+      plane_nibbles(w[k], n0, n1, nv, nu);
       b0 |= n0 << (4 * k);
       b1 |= n1 << (4 * k);
       bv |= nv << (4 * k);
+      bu |= nu << (4 * k);
     }
     const uint32_t o0 = __shfl_down_sync(0xFFFFFFFFu, b0, 1);
     const uint32_t o1 = __shfl_down_sync(0xFFFFFFFFu, b1, 1);
     const uint32_t ov = __shfl_down_sync(0xFFFFFFFFu, bv, 1);
+    const uint32_t ou = __shfl_down_sync(0xFFFFFFFFu, bu, 1);
     const uint64_t blk = sp * 16u + (lane >> 1);
     if (!(lane & 1u) && blk < nblocks)
-      out[blk] = make_uint4(b0 | (o0 << 16), b1 | (o1 << 16), bv | (ov << 16), 0u);
+      out[blk] = make_uint4(b0 | (o0 << 16), b1 | (o1 << 16), bv | (ov << 16), bu | (ou << 16));
   }
 }
 
-// Number of positions i in [0, len) with a[i] != b[i], stopping once above
-// `limit` (bounded_hamming, src/alignment/mod.rs:764-776). Warp-cooperative.
-__device__ __forceinline__ uint32_t warp_bounded_hamming(const uint8_t* a, const uint8_t* b,
-                                                         uint32_t len, uint32_t limit,
-                                                         uint32_t lane) {
-  uint32_t m = 0;
-  for (uint32_t c = 0; c < len; c += 32u) {
-    const uint32_t i = c + lane;
-    const bool ne = i < len && ldb(a, i) != ldb(b, i);
-    m += __popc(__ballot_sync(0xFFFFFFFFu, ne));
-    if (m > limit) break;
-  }
-  return m;
-}
-
-// spectral_hit_is_certified (src/alignment/mod.rs:688-762), warp-cooperative.
-__device__ bool warp_certify(const uint8_t* read, const uint8_t* ref, uint32_t len, uint32_t mism,
-                             uint32_t second, uint32_t max_mism, bool strict, uint32_t lane) {
-  if (mism > max_mism) return false;
-  if (second != kNoKey && second <= mism + 1u) return false;
-  if (mism == 0) return true;
-  if (mism > 2) return false;
-  uint32_t n = 0, pos0 = 0xFFFFFFFFu, pos1 = 0xFFFFFFFFu;
-  for (uint32_t c = 0; c < len; c += 32u) {
-    const uint32_t i = c + lane;
-    const bool ne = i < len && ldb(read, i) != ldb(ref, i);
-    uint32_t b = __ballot_sync(0xFFFFFFFFu, ne);
-    while (b) {
-      const uint32_t at = c + (uint32_t)(__ffs(b) - 1);
-      if (n == 0) pos0 = at;
-      else if (n == 1) pos1 = at;
-      ++n;
-      b &= b - 1u;
-    }
-  }
-  if (n != mism) return false;
-  const uint32_t edge = min(len, 8u);
-  if (pos0 < edge || pos0 + edge >= len) return false;
-  if (n == 2 && (pos1 < edge || pos1 + edge >= len)) return false;
-  if (n == 2 && (pos1 > pos0 ? pos1 - pos0 : 0u) <= 4u) return false;
-  const uint32_t p = pos0;
-  const uint32_t suffix = len > p + 1u ? len - (p + 1u) : 0u;
-  const uint32_t min_suffix = strict ? 4u : 8u;
-  if (suffix >= min_suffix) {
-    if (warp_bounded_hamming(read + p + 1, ref + p, len - p - 1u, 1u, lane) <= 1u) return false;
-    if (warp_bounded_hamming(read + p, ref + p + 1, len - p - 1u, 1u, lane) <= 1u) return false;
-    if (strict && suffix >= 6u) {
-      if (warp_bounded_hamming(read + p + 2, ref + p, len - p - 2u, 1u, lane) <= 1u) return false;
-      if (warp_bounded_hamming(read + p, ref + p + 2, len - p - 2u, 1u, lane) <= 1u) return false;
-    }
-  }
-  return true;
-}
-
-// spectral_hit_is_certified (src/alignment/mod.rs:688-762) for one lane's pair.
+// spectral_hit_is_certified (src/alignment/mod.rs:688-762) for one lane's pair, on the
+// bytes: pairs with lower-case bases (sieve_certified does the others).
 __device__ __forceinline__ uint32_t lane_bounded_hamming(const uint8_t* a, const uint8_t* b,
                                                          uint32_t len, uint32_t limit) {
   uint32_t m = 0;
@@ -266,23 +218,23 @@ __device__ __forceinline__ void warp_append(bool take, uint32_t value, uint32_t*
 template <int RWMAX>
 __device__ __forceinline__ bool sieve_certify(const DevPairs& P, const VerifyDev& V, uint32_t p,
                                               uint32_t q, LaneSieve& so) {
-  so = sieve_lane<RWMAX>(P.read_planes, P.read_off[p], q, P.win_planes, P.win_off[p],
-                         P.win_len[p]);
   const uint32_t thr = sieve_threshold_for(V.sieve_threshold, q);
-  const bool cert = so.hit && so.mism <= thr &&
-                    lane_certify(P.read_seq + P.read_off[p], P.win_seq + P.win_off[p] + so.shift,
-                                 q, so.mism, so.second, thr, V.cert_strict != 0);
+  so = sieve_lane<RWMAX>(P.read_planes, P.read_off[p], q, P.win_planes, P.win_off[p],
+                         P.win_len[p], thr, V.cert_strict != 0);
+  const bool cert =
+      so.cert == 1u ||
+      (so.cert == 2u && lane_certify(P.read_seq + P.read_off[p], P.win_seq + P.win_off[p] + so.shift,
+                                     q, so.mism, so.second, thr, V.cert_strict != 0));
   if (cert) write_certified(V, p, q, so);
   return cert;
 }
 
 // Stage 1 of the composed path when detail rows are asked for or the filter is
-// off: sieve + certificate of every pair, then the 4-gram filter, one lane per pair.
+// off: sieve + certificate of every pair, then the block filter, one lane per pair.
 template <int RWMAX>
 __global__ void __launch_bounds__(256) verify_sieve_kernel(DevPairs P, VerifyDev V) {
-  __shared__ uint32_t qset[8][16 * 32];  // per warp: 4-gram bitmap [word][lane]
-  const uint32_t lane = threadIdx.x & 31u;
-  uint32_t* myset = &qset[threadIdx.x >> 5][lane];
+  __shared__ uint32_t qset[8][32 * kQgramWords];  // per warp: a 5-gram set per read
+  uint32_t* sets = qset[threadIdx.x >> 5];
   const uint32_t stride = gridDim.x * blockDim.x;
   for (uint32_t base = blockIdx.x * blockDim.x; base < P.n; base += stride) {
     const uint32_t p = base + threadIdx.x;
@@ -291,7 +243,7 @@ __global__ void __launch_bounds__(256) verify_sieve_kernel(DevPairs P, VerifyDev
     uint32_t q = 0;
     if (valid) {
       q = P.read_len[p];
-      LaneSieve so{false, 0, 0, 0xFFFFFFFFu};
+      LaneSieve so{false, 0, 0, 0xFFFFFFFFu, 0u};
       cert = sieve_certify<RWMAX>(P, V, p, q, so);
       if (V.detail) {
         kira_verify_detail dt;
@@ -304,76 +256,90 @@ __global__ void __launch_bounds__(256) verify_sieve_kernel(DevPairs P, VerifyDev
       }
       if (!cert) V.sw_offset[p] = so.hit ? (int32_t)so.shift : 0;
     }
-    // Exact 4-gram prefilter: a pair it rejects is a Myers None (same result).
+    // Exact block filter: a pair it rejects is a Myers None (same result).
     bool gone = false;
-    if (valid && !cert && V.qgram) {
-      const uint32_t k = myers_k_for(V.myers_k, q);
-      gone = qgram4_reject(P.read_planes, P.read_off[p], q, P.win_planes, P.win_off[p],
-                           P.win_len[p], k, myset);
+    if (V.qgram) {
+      const int32_t need = valid ? qgram_need(q, myers_k_for(V.myers_k, q)) : 0;
+      gone = qgram_outcome(valid && !cert, P.read_planes, valid ? P.read_off[p] : 0u, q,
+                           P.win_planes, valid ? P.win_off[p] : 0u, valid ? P.win_len[p] : 0u,
+                           need, need, sets) != 0u;
       if (gone) write_myers_reject(V, p);
     }
     warp_append(valid && !cert && !gone, p, V.counters + 0, V.myers_list);
   }
 }
 
-// Stage 1, filter first (no detail rows): the 4-gram count of every pair decides
-// two things. Myers rejects the pair when count < m - 3 - 4k (qgram.cuh). And the
-// certificate needs a shift with at most min(threshold, 2) mismatches
-// (lane_certify): a shift with d mismatches leaves at least m - 3 - 4d read
-// 4-grams untouched, each found verbatim in the window, so count < m - 3 -
-// 4 min(threshold, 2) proves no shift certifies. A pair below both bounds is a
-// Myers reject whatever its sieve says, and its sieve is never run; the others go
-// to verify_sieve_list_kernel, tagged when the count already rejects them unless
+// Resident blocks of the filter on an SM (32 KB of sets each): its grid, so that none
+// waits for a second wave. (A fuller SM is slower: past 4 blocks the sets leave the
+// plane loads too little L1.)
+constexpr int kFilterBlocks = 4;
+
+// Stage 1, filter first (no detail rows): the block count of every pair decides
+// two things. Myers rejects the pair when the count is below the bound for k edits
+// (qgram.cuh). And the certificate needs a shift with at most min(threshold, 2)
+// mismatches (lane_certify): that shift is an alignment with as many edits, so a count
+// below the bound for min(threshold, 2) proves no shift certifies. A pair below both
+// bounds is a Myers reject whatever its sieve says, and its sieve is never run; the others
+// go to verify_sieve_list_kernel, tagged when the count already rejects them unless
 // they certify. Rows are those of verify_sieve_kernel.
-__global__ void __launch_bounds__(256) verify_filter_kernel(DevPairs P, VerifyDev V) {
-  __shared__ uint32_t qset[8][16 * 32];
-  const uint32_t lane = threadIdx.x & 31u;
-  uint32_t* myset = &qset[threadIdx.x >> 5][lane];
+__global__ void __launch_bounds__(256, kFilterBlocks) verify_filter_kernel(DevPairs P,
+                                                                           VerifyDev V) {
+  __shared__ uint32_t qset[8][32 * kQgramWords];
+  uint32_t* sets = qset[threadIdx.x >> 5];
   const uint32_t stride = gridDim.x * blockDim.x;
   for (uint32_t base = blockIdx.x * blockDim.x; base < P.n; base += stride) {
     const uint32_t p = base + threadIdx.x;
     const bool valid = p < P.n;
-    uint32_t outcome = 0;
+    int32_t lo = 0, hi = 0;
+    uint32_t q = 0;
     if (valid) {
-      const uint32_t q = P.read_len[p];
-      const int32_t thr2 = (int32_t)min(sieve_threshold_for(V.sieve_threshold, q), 2u);
-      const int32_t hi = (int32_t)q - 3 - 4 * (int32_t)myers_k_for(V.myers_k, q);
-      const int32_t lo = min(hi, (int32_t)q - 3 - 4 * thr2);
-      outcome = qgram4_outcome(P.read_planes, P.read_off[p], q, P.win_planes, P.win_off[p],
-                               P.win_len[p], lo, hi, myset);
-      if (outcome == 2u) write_myers_reject(V, p);
+      q = P.read_len[p];
+      const uint32_t thr2 = min(sieve_threshold_for(V.sieve_threshold, q), 2u);
+      const uint32_t k = myers_k_for(V.myers_k, q);
+      hi = qgram_need(q, k);
+      lo = qgram_need(q, max(k, thr2));
     }
+    const uint32_t outcome = qgram_outcome(
+        valid, P.read_planes, valid ? P.read_off[p] : 0u, q, P.win_planes,
+        valid ? P.win_off[p] : 0u, valid ? P.win_len[p] : 0u, lo, hi, sets);
+    if (outcome == 2u) write_myers_reject(V, p);
     warp_append(valid && outcome != 2u, p | (outcome == 1u ? 0x80000000u : 0u), V.sieve_count,
                 V.sieve_list);
   }
 }
 
 // Stage 1, second pass: sieve + certificate of the listed pairs; a pair that does
-// not certify is a Myers reject when tagged, else it goes to the Myers list with
-// its sieve shift as the banded-SW offset.
+// not certify is a Myers reject when tagged, else it goes to the Myers list -- or past
+// it, when its best shift already has at most k mismatches -- with that shift as the
+// banded-SW offset. (The Myers stage of 2M pairs is left with reads whose indel spoils
+// every shift.)
 template <int RWMAX>
-__global__ void __launch_bounds__(256, 4) verify_sieve_list_kernel(DevPairs P, VerifyDev V) {
+__global__ void __launch_bounds__(256, RWMAX <= 5 ? 3 : 2) verify_sieve_list_kernel(DevPairs P, VerifyDev V) {
   const uint32_t count = *V.sieve_count;
   const uint32_t stride = gridDim.x * blockDim.x;
   for (uint32_t base = blockIdx.x * blockDim.x; base < count; base += stride) {
     const uint32_t idx = base + threadIdx.x;
     const bool valid = idx < count;
-    bool to_myers = false;
+    bool to_myers = false, to_sw = false;
     uint32_t p = 0;
     if (valid) {
       const uint32_t e = V.sieve_list[idx];
       p = e & 0x7FFFFFFFu;
-      LaneSieve so{false, 0, 0, 0xFFFFFFFFu};
+      LaneSieve so{false, 0, 0, 0xFFFFFFFFu, 0u};
       if (!sieve_certify<RWMAX>(P, V, p, P.read_len[p], so)) {
         if (e >> 31) {
           write_myers_reject(V, p);
         } else {
           V.sw_offset[p] = so.hit ? (int32_t)so.shift : 0;
-          to_myers = true;
+          // An ungapped alignment with at most k mismatches is one with at most k
+          // edits: Myers would accept the pair, and its distance is not asked for.
+          to_sw = so.hit && so.mism <= myers_k_for(V.myers_k, P.read_len[p]);
+          to_myers = !to_sw;
         }
       }
     }
     warp_append(to_myers, p, V.counters + 0, V.myers_list);
+    warp_append(to_sw, V.sw_base + p, V.sw_count, V.sw_list);
   }
 }
 
@@ -409,14 +375,13 @@ __device__ void myers_warp(const DevPairs& P, const MyersLaunch& M, uint32_t bas
   __syncwarp();
   uint32_t dist = 0, endp = 0;
   bool hit = false;
-  const bool uniform = __all_sync(0xFFFFFFFFu, !valid || (m + 31u) / 32u == (uint32_t)L);
   if (valid) {
     const uint32_t n = P.win_len[pair];
     const uint32_t k = M.per_pair_k ? myers_k_for(M.k, m) : (uint32_t)M.k;
-    hit = uniform ? myers_lane<L, true>(m, n, k, sm, P.win_planes, P.win_off[pair], lane, dist,
-                                        endp)
-                  : myers_lane<L, false>(m, n, k, sm, P.win_planes, P.win_off[pair], lane, dist,
-                                         endp);
+    // Without detail rows the cascade asks only whether the pair is within k.
+    hit = M.cascade && !M.detail
+              ? myers_lane<L, false>(m, n, k, sm, P.win_planes, P.win_off[pair], lane, dist, endp)
+              : myers_lane<L, true>(m, n, k, sm, P.win_planes, P.win_off[pair], lane, dist, endp);
   }
   __syncwarp();
   if (M.cascade) {
@@ -978,7 +943,8 @@ cudaError_t launch_verify_sieve(const DevPairs& P, const VerifyDev& V, uint32_t 
   if (V.sieve_list && !V.detail && V.qgram && P.n < 0x80000000u) {
     cudaError_t e = cudaMemsetAsync(V.sieve_count, 0, 4, st);
     if (e != cudaSuccess) return e;
-    (verify_filter_kernel<<<blocks, 256, 0, st>>>(P, V), count_launch());
+    (verify_filter_kernel<<<grid_for(P.n, 256, sms * kFilterBlocks), 256, 0, st>>>(P, V),
+     count_launch());
     if (rw <= 5) (verify_sieve_list_kernel<5><<<blocks, 256, 0, st>>>(P, V), count_launch());
     else if (rw <= 8) (verify_sieve_list_kernel<8><<<blocks, 256, 0, st>>>(P, V), count_launch());
     else (verify_sieve_list_kernel<16><<<blocks, 256, 0, st>>>(P, V), count_launch());

@@ -8,15 +8,23 @@
 // nothing; pattern bytes outside ACGT set no Peq bit.
 //
 // B200 mapping: the bit vector is held as L 32-bit limbs in registers (the
-// reference uses 64-bit blocks; bits below m never depend on bits above m, so
-// the limb width does not change any result). One lane per pair:
+// reference uses 64-bit blocks; the limb width does not change any result). One lane
+// per pair:
 //   * pattern and text come from the 2-bit + valid plane arenas (planes.cuh):
 //     one 32-base word is two 16-byte loads and a funnel shift, no cross-lane work;
+//   * the pattern ends at the top bit of the top limb, whatever its length: the bits
+//     below its first base are rows that match every base and start with no vertical
+//     difference, so they stay rows of zeros -- the boundary the first base needs. No
+//     limb is masked and the score change of a column is the top limb's top bit, for
+//     patterns of different lengths in one warp alike (per-limb masks and a per-limb
+//     choice of the top one were a third of the work: 131k pairs of 100-250 bases);
 //   * Peq lives in shared memory as [k][code][lane] with code 4 = "matches
-//     nothing" (all zero), so every per-lane read is bank-conflict-free.
+//     nothing" (only the rows below the pattern), so every per-lane read is
+//     bank-conflict-free.
 //   * Per column and limb: one LDS for Eq (instead of a 4-way select), the
 //     (Eq & VP) + VP carry chain on the PTX carry flag (add.cc / addc), and one
-//     funnel shift for each of the HP / HN shifts across limbs.
+//     funnel shift for each of the HP / HN shifts across limbs: ten operations on the
+//     ALU pipe, which bounds it.
 #pragma once
 
 #include "addchain.cuh"
@@ -30,30 +38,43 @@ struct MyersSmem {
   uint32_t* peq;  // [L][5][32]
 };
 
+// Rows of limb k below a pattern of m bases that ends at bit 32L - 1.
+template <int L>
+__device__ __forceinline__ uint32_t myers_below(int k, uint32_t m) {
+  const int32_t lo = 32 * k - (int32_t)(32u * L - m);  // pattern position of the limb's bit 0
+  return lo <= -32 ? 0xFFFFFFFFu : lo < 0 ? (1u << -lo) - 1u : 0u;
+}
+
 // Builds this lane's Peq columns from the pattern's plane words (no cross-lane
-// work): eq_A = ~b1 & ~b0 & valid, ... for the bases below m.
+// work): eq_A = ~b1 & ~b0 & valid, ... and the rows below the pattern everywhere.
 template <int L>
 __device__ __forceinline__ void myers_build_peq(const uint4* __restrict__ planes, uint64_t pos,
                                                 uint32_t m, uint32_t lane, MyersSmem sm) {
 #pragma unroll
   for (int k = 0; k < L; ++k) {
-    const PlaneWord pw = plane_word_at(planes, pos + 32u * k);
-    const uint32_t base = 32u * (uint32_t)k;
-    const uint32_t lm = base < m ? low_mask(m - base) : 0u;
-    const uint32_t v = pw.v & lm;
+    const int32_t lo = 32 * k - (int32_t)(32u * L - m);
+    PlaneWord pw{0u, 0u, 0u};
+    if (lo > -32) {
+      pw = plane_word_at(planes, pos + (uint32_t)max(lo, 0));
+      if (lo < 0) {
+        pw.b0 <<= -lo;
+        pw.b1 <<= -lo;
+        pw.v <<= -lo;
+      }
+    }
+    const uint32_t below = myers_below<L>(k, m);
     uint32_t* col = sm.peq + (uint32_t)k * 160u + lane;
-    col[0] = ~pw.b1 & ~pw.b0 & v;
-    col[32] = ~pw.b1 & pw.b0 & v;
-    col[64] = pw.b1 & ~pw.b0 & v;
-    col[96] = pw.b1 & pw.b0 & v;
-    col[128] = 0u;
+    col[0] = (~pw.b1 & ~pw.b0 & pw.v) | below;
+    col[32] = (~pw.b1 & pw.b0 & pw.v) | below;
+    col[64] = (pw.b1 & ~pw.b0 & pw.v) | below;
+    col[96] = (pw.b1 & pw.b0 & pw.v) | below;
+    col[128] = below;
   }
 }
 
-// Runs the recurrence for this lane's pair. Returns true with (dist, end) on a
-// hit <= max_k. UNIFORM: every lane of the warp has ceil(m / 32) == L (no limb
-// masks below the top limb). Otherwise limbs above the pattern stay masked to 0.
-template <int L, bool UNIFORM>
+// Runs the recurrence for this lane's pair (m <= 32 L). Returns true on a hit <= max_k;
+// with WHERE, (dist, end) of the best column, else as soon as one column is a hit.
+template <int L, bool WHERE>
 __device__ __forceinline__ bool myers_lane(uint32_t m, uint32_t n, uint32_t max_k,
                                            MyersSmem sm, const uint4* __restrict__ tplanes,
                                            uint64_t tpos, uint32_t lane, uint32_t& dist,
@@ -68,55 +89,28 @@ __device__ __forceinline__ bool myers_lane(uint32_t m, uint32_t n, uint32_t max_
     end_pos = 0;
     return m <= max_k;
   }
-  const uint32_t nl = (m + 31u) / 32u;
-  const uint32_t top_used = m - 32u * (nl - 1u);
-  const uint32_t top_mask = top_used == 32u ? 0xFFFFFFFFu : ((1u << top_used) - 1u);
-  const uint32_t high = 1u << (top_used - 1u);
-  uint32_t vp[L], vn[L], lm[L];
+  uint32_t vp[L], vn[L];
 #pragma unroll
   for (int k = 0; k < L; ++k) {
-    if (UNIFORM)
-      lm[k] = k + 1 < L ? 0xFFFFFFFFu : top_mask;
-    else
-      lm[k] = (uint32_t)k + 1u < nl ? 0xFFFFFFFFu : ((uint32_t)k + 1u == nl ? top_mask : 0u);
-    vp[k] = lm[k];
+    vp[k] = ~myers_below<L>(k, m);
     vn[k] = 0u;
   }
   const uint32_t* peq = sm.peq + lane;
   uint32_t err = m, best = m, pos = 0;
-  // Software pipelined over the text: the Peq words of column j + 1 are loaded while
-  // column j is computed, and the text plane word of the next 32 columns one block
-  // ahead, so neither load's latency sits on the column-to-column chain.
-  // Column code: 0-3 for ACGT, 4 (an all-zero Peq row) for any other base.
-  auto code_at = [](uint32_t bit, const PlaneWord& w) {
-    return ((w.v >> bit) & 1u) ? (((w.b0 >> bit) & 1u) | (((w.b1 >> bit) & 1u) << 1)) : 4u;
+  if (!WHERE && m <= max_k) return true;
+  // Column code: 0-3 for ACGT, 4 (the rows below the pattern alone) for any other base.
+  auto load = [&](uint32_t b0, uint32_t b1, uint32_t v, uint32_t (&eq)[L]) {
+    const uint32_t* pc = peq + ((v & 1u) ? ((b0 & 1u) | ((b1 & 1u) << 1)) : 4u) * 32u;
+#pragma unroll
+    for (int k = 0; k < L; ++k) eq[k] = pc[k * 160];
   };
-  PlaneWord cw = plane_word_at(tplanes, tpos);
-  PlaneWord nw = n > 32u ? plane_word_at(tplanes, tpos + 32u) : cw;
-  uint32_t eqn[L];
-  {
-    const uint32_t* pc = peq + code_at(0u, cw) * 32u;
+  uint32_t j = 0;  // columns done
+  auto column = [&](const uint32_t (&eq)[L]) {
+    uint32_t av[L], sum[L];
 #pragma unroll
-    for (int k = 0; k < L; ++k) eqn[k] = pc[k * 160];
-  }
-  for (uint32_t j = 0; j < n; ++j) {
-    uint32_t eq[L], av[L], sum[L];
-#pragma unroll
-    for (int k = 0; k < L; ++k) {
-      eq[k] = eqn[k];
-      av[k] = eq[k] & vp[k];
-    }
-    if ((j & 31u) == 31u) {  // column j + 1 opens the next block of 32
-      cw = nw;
-      if (j + 33u < n) nw = plane_word_at(tplanes, tpos + j + 33u);
-    }
-    if (j + 1u < n) {
-      const uint32_t* pc = peq + code_at((j + 1u) & 31u, cw) * 32u;
-#pragma unroll
-      for (int k = 0; k < L; ++k) eqn[k] = pc[k * 160];
-    }
+    for (int k = 0; k < L; ++k) av[k] = eq[k] & vp[k];
     add_chain<L>(av, vp, sum);
-    uint32_t hp_prev = 0, hn_prev = 0, hp_top = 0, hn_top = 0;
+    uint32_t hp_prev = 0, hn_prev = 0;
 #pragma unroll
     for (int k = 0; k < L; ++k) {
       const uint32_t vpk = vp[k], vnk = vn[k];
@@ -127,28 +121,51 @@ __device__ __forceinline__ bool myers_lane(uint32_t m, uint32_t n, uint32_t max_
       const uint32_t hns = k ? __funnelshift_l(hn_prev, hn, 1) : (hn << 1);
       hp_prev = hp;
       hn_prev = hn;
-      vp[k] = (hns | ~(d0 | hps)) & lm[k];
-      vn[k] = (d0 & hps) & lm[k];
-      if (UNIFORM) {
-        if (k == L - 1) {
-          hp_top = hp;
-          hn_top = hn;
-        }
-      } else if ((uint32_t)k + 1u == nl) {
-        hp_top = hp;
-        hn_top = hn;
+      vp[k] = hns | ~(d0 | hps);
+      vn[k] = d0 & hps;
+    }
+    err = err + (hp_prev >> 31) - (hn_prev >> 31);
+    ++j;
+    if (WHERE) {
+      if (err <= best) {
+        best = err;
+        pos = j;
       }
+    } else {
+      best = min(best, err);
     }
-    err += (hp_top & high) ? 1u : 0u;
-    err -= (hn_top & high) ? 1u : 0u;
-    if (err <= best) {
-      best = err;
-      pos = j + 1u;
+  };
+  // Four columns a step: their Peq words are loaded together, ahead of the chain from
+  // column to column, and the exits are tested once. The text plane word of the next 32
+  // columns is loaded a block ahead.
+  PlaneWord nw = plane_word_at(tplanes, tpos);
+  for (uint32_t base = 0; base < n; base += 32u) {
+    PlaneWord cw = nw;
+    if (base + 32u < n) nw = plane_word_at(tplanes, tpos + base + 32u);
+    uint32_t left = min(32u, n - base);
+    for (; left >= 4u; left -= 4u) {
+      uint32_t eq[4][L];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) load(cw.b0 >> t, cw.b1 >> t, cw.v >> t, eq[t]);
+      cw.b0 >>= 4;
+      cw.b1 >>= 4;
+      cw.v >>= 4;
+#pragma unroll
+      for (int t = 0; t < 4; ++t) column(eq[t]);
+      if (!WHERE && best <= max_k) return true;
+      // No later column can come down to k (myers.rs:194).
+      if (best > max_k && err > max_k + (n - j)) return false;
     }
-    const uint32_t rem = n - 1u - j;
-    const uint32_t sat = err > rem ? err - rem : 0u;
-    if (best > max_k && sat > max_k) return false;  // myers.rs:194
+    for (; left; --left) {
+      uint32_t eq[L];
+      load(cw.b0, cw.b1, cw.v, eq);
+      cw.b0 >>= 1;
+      cw.b1 >>= 1;
+      cw.v >>= 1;
+      column(eq);
+    }
   }
+  if (!WHERE) return best <= max_k;
   if (best <= max_k) {
     dist = best;
     end_pos = pos;

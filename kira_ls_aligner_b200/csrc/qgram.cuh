@@ -1,29 +1,31 @@
-// qgram.cuh -- exact 4-gram prefilter in front of the Myers stage.
+// qgram.cuh -- exact block filter in front of the Myers stage.
 //
 // The Myers stage (bounded_edit_distance, src/alignment/myers.rs:47-70) answers
-// None unless the read aligns to some substring T' of the window with at most k
-// edits. Each edit (substitution, deletion from the read, or insertion between
-// two read bases) touches at most four of the read's m - 3 overlapping 4-grams;
-// every untouched read 4-gram occurs verbatim in T', hence in the window. So
+// None unless the read (m bases) aligns to some substring T' of the window with at
+// most k edits. T' has at least m - k bases, so of the window's blocks [5j, 5j + 5) at
+// least floor((m - k - 4) / 5) lie inside it, and one edit (a substitution, a window
+// base without a partner, or read bases between two window bases) touches at most one
+// of them; every untouched block occurs verbatim in the read. So
 //
-//     ed <= k  implies  #{p : read[p, p+4) occurs in the window} >= m - 3 - 4k.
+//     ed <= k  implies  #{j : window block j occurs in the read} >= (m - k - 4) / 5 - k.
 //
 // A pair whose count is below that bound is a Myers None for certain, and the
 // filter answers exactly that (the same MYERS_REJECT result and detail). Bases
-// outside ACGT match nothing in Myers: a read 4-gram containing one can never
-// be untouched and is not counted, and window 4-grams containing one are not
-// inserted. The filter only ever removes pairs Myers would reject, so every
-// output is unchanged; survivors still run Myers.
+// outside ACGT match nothing in Myers: each costs an edit of its own, so a block (or a
+// read 5-gram) that contains one is left out. The filter only ever removes pairs Myers
+// would reject, so every output is unchanged; survivors still run Myers.
 //
-// Lane-per-pair: the window's 4-gram set is a 256-bit bitmap per lane in shared
-// memory, 16 words of 16 used bits laid out [word][lane] (each lane owns one
-// bank); bases come from the 2-bit + valid plane arenas, one 32-base word at a
-// time. A 4-gram is its four bit-1 plane bits (the word) and its four bit-0 plane
-// bits (the bit in it), each one bit-field extract, the previous word supplying
-// the first three bases of a word; the positions whose four bases are all valid
-// come from one AND of shifted valid masks per word. An insert is one shared-memory
-// atomic OR (each lane owns its column, so nothing contends). Window and read use
-// the same index, so the count is the count.
+// Why blocks of 5 and the read's set: the set of a read's 5-grams is 1024 bits, and a
+// random window block is in it with probability about 145 / 1024 at 150 bases, 6.6 of
+// 50 blocks, against a bound of 19 at k = 8. Only n / 5 look-ups per pair remain (a
+// filter on all 4-grams, the window's set against the read's grams, took 247 inserts and
+// 147 look-ups), and the candidates of one read, which lie next to each other in a
+// batch, share one set: the lanes of a warp that hold the same read build it together.
+// 2M pairs of 150 / 250 bp, 8 candidates a read.
+//
+// A set is 32 words in shared memory, contiguous, one per distinct read of the warp: a
+// 5-gram's code-bit-1 bits choose the word and its code-bit-0 bits the bit in it, both
+// straight from the plane words.
 #pragma once
 
 #include "common.cuh"
@@ -31,91 +33,107 @@
 
 namespace kira {
 
-// Bits [b - 3, b] of the base stream ... prev | cur (b in 0..31, compile-time).
-template <int B>
-__device__ __forceinline__ uint32_t qgram_nibble(uint32_t prev, uint32_t cur) {
-  if constexpr (B >= 3) return (cur >> (B - 3)) & 0xFu;
-  else return __funnelshift_r(prev, cur, 29 + B) & 0xFu;
+constexpr uint32_t kQgram = 5, kQgramWords = 32;
+
+// The bound above (<= 0: the filter proves nothing).
+__device__ __forceinline__ int32_t qgram_need(uint32_t m, uint32_t k) {
+  const int32_t inside = (int32_t)m - (int32_t)k - (int32_t)(kQgram - 1u);
+  return inside > 0 ? inside / (int32_t)kQgram - (int32_t)k : 0;
 }
 
-// Positions of a word whose 4-gram (this base and the three before) is all ACGT.
-__device__ __forceinline__ uint32_t qgram_valid4(uint32_t pv, uint32_t v, uint32_t lim) {
-  uint32_t v4 = v & __funnelshift_l(pv, v, 1) & __funnelshift_l(pv, v, 2) &
-                __funnelshift_l(pv, v, 3);
-  return lim < 32u ? v4 & ((1u << lim) - 1u) : v4;
+// Positions whose kQgram bases from there on are all set in v (32 bases).
+__device__ __forceinline__ uint32_t qgram_valid(uint32_t v) {
+  return v & (v >> 1) & (v >> 2) & (v >> 3) & (v >> 4);
 }
 
-
-// Where the count of read 4-grams found in the window falls against two bounds
-// lo <= hi: 0 when count >= hi, 1 when lo <= count < hi, 2 when count < lo; the
-// read walk stops as soon as that is decided. With hi <= 0 or a window of fewer
-// than four bases the answer is 0 (nothing is proved). `set` points at this
-// lane's column of a [16][32] word bitmap in shared memory.
-__device__ __forceinline__ uint32_t qgram4_outcome(const uint4* __restrict__ rplanes,
-                                                   uint64_t rpos, uint32_t m,
-                                                   const uint4* __restrict__ wplanes,
-                                                   uint64_t wpos, uint32_t n, int32_t lo,
-                                                   int32_t hi, uint32_t* set) {
-  if (hi <= 0 || n < 4u) return 0u;
+// Where the count of this lane's window blocks found in its read falls against two
+// bounds lo <= hi: 0 when count >= hi, 1 when lo <= count < hi, 2 when count < lo. All 32
+// lanes call; a lane with `active` false or hi <= 0 gets 0 (nothing is proved). `sets`:
+// the warp's 32 x kQgramWords words.
+__device__ __forceinline__ uint32_t qgram_outcome(bool active, const uint4* __restrict__ rplanes,
+                                                  uint64_t rpos, uint32_t m,
+                                                  const uint4* __restrict__ wplanes, uint64_t wpos,
+                                                  uint32_t n, int32_t lo, int32_t hi,
+                                                  uint32_t* sets) {
+  constexpr uint32_t kAll = 0xFFFFFFFFu;
+  const uint32_t lane = threadIdx.x & 31u;
+  active = active && hi > 0 && m >= kQgram;
+  if (!__any_sync(kAll, active)) return 0u;
+  // Lanes with the same read (an inactive lane is alone: its key is no arena offset).
+  const uint32_t same = __match_any_sync(kAll, active ? rpos : ~(uint64_t)lane) &
+                        __match_any_sync(kAll, m);
+  const uint32_t leader = (uint32_t)(__ffs(same) - 1), size = (uint32_t)__popc(same);
+  const uint32_t rank = (uint32_t)__popc(same & ((1u << lane) - 1u));
+  uint32_t* set = sets + leader * kQgramWords;
+  if (active) {
+    for (uint32_t w = rank; w < kQgramWords; w += size) set[w] = 0u;
+  }
+  __syncwarp();
+  if (active) {
+    constexpr uint32_t kUnit = 16;  // 5-gram starts a step: one plane word
+    const uint32_t grams = m - (kQgram - 1u);
+    for (uint32_t s = rank * kUnit; s < grams; s += size * kUnit) {
+      const PlaneWord pw = plane_word_at(rplanes, rpos + s);
+      const uint32_t ok = qgram_valid(pw.v) & low_mask(min(grams - s, kUnit));
+      if (ok == low_mask(kUnit)) {
 #pragma unroll
-  for (int w = 0; w < 16; ++w) set[w * 32] = 0u;
-  uint32_t p0 = 0, p1 = 0, pv = 0;
-  for (uint32_t blk = 0; blk * 32u < n; ++blk) {
-    const PlaneWord pw = plane_word_at(wplanes, wpos + 32u * blk);
-    const uint32_t v4 = qgram_valid4(pv, pw.v, min(32u, n - 32u * blk));
-#define KIRA_QG_INS(B) \
-  atomicOr(&set[qgram_nibble<(B)>(p1, pw.b1) * 32u], 1u << qgram_nibble<(B)>(p0, pw.b0));
-#define KIRA_QG_SET(B) \
-  if ((v4 >> (B)) & 1u) KIRA_QG_INS(B)
-#define KIRA_QG_ALL(M)                                                                   \
-  M(0) M(1) M(2) M(3) M(4) M(5) M(6) M(7) M(8) M(9) M(10) M(11) M(12) M(13) M(14) M(15) \
-  M(16) M(17) M(18) M(19) M(20) M(21) M(22) M(23) M(24) M(25) M(26) M(27) M(28) M(29)   \
-  M(30) M(31)
-    // A word whose 32 positions are all valid (no N near it) skips the per-position tests.
-    if (v4 == 0xFFFFFFFFu) {
-      KIRA_QG_ALL(KIRA_QG_INS)
-    } else {
-      KIRA_QG_ALL(KIRA_QG_SET)
+        for (uint32_t t = 0; t < kUnit; ++t)
+          atomicOr(&set[(pw.b1 >> t) & 31u], 1u << ((pw.b0 >> t) & 31u));
+      } else {
+#pragma unroll
+        for (uint32_t t = 0; t < kUnit; ++t)
+          if ((ok >> t) & 1u) atomicOr(&set[(pw.b1 >> t) & 31u], 1u << ((pw.b0 >> t) & 31u));
+      }
     }
-#undef KIRA_QG_SET
-#undef KIRA_QG_INS
-    p0 = pw.b0, p1 = pw.b1, pv = pw.v;
   }
-  int32_t count = 0;
-  p0 = p1 = pv = 0;
-  for (uint32_t blk = 0; blk * 32u < m; ++blk) {
-    const PlaneWord pw = plane_word_at(rplanes, rpos + 32u * blk);
-    const uint32_t lim = min(32u, m - 32u * blk);
-    const uint32_t v4 = qgram_valid4(pv, pw.v, lim);
-#define KIRA_QG_HIT(B) \
-  count += (int32_t)((set[qgram_nibble<(B)>(p1, pw.b1) * 32u] >> qgram_nibble<(B)>(p0, pw.b0)) & 1u);
-#define KIRA_QG_COUNT(B) \
-  if ((v4 >> (B)) & 1u) KIRA_QG_HIT(B)
-    if (v4 == 0xFFFFFFFFu) {
-      KIRA_QG_ALL(KIRA_QG_HIT)
-    } else {
-      KIRA_QG_ALL(KIRA_QG_COUNT)
+  __syncwarp();
+  uint32_t count = 0;
+  if (active) {
+    // 160 bases (5 plane words) hold 32 blocks.
+    for (uint32_t base = 0; base + kQgram <= n; base += 160u) {
+      uint32_t b0[6], b1[6], all = 0xFFFFFFFFu, v[6];
+#pragma unroll
+      for (int k = 0; k < 5; ++k) {
+        PlaneWord pw{0u, 0u, 0xFFFFFFFFu};  // past the window: no block counts there
+        if (base + 32u * k < n) pw = plane_word_at(wplanes, wpos + base + 32u * k);
+        b0[k] = pw.b0;
+        b1[k] = pw.b1;
+        v[k] = pw.v;
+        all &= pw.v;
+      }
+      b0[5] = b1[5] = v[5] = 0u;
+      const uint32_t blocks = min((n - base) / kQgram, 32u);
+      uint32_t hits = 0;  // block j at bit 31 - j
+#pragma unroll
+      for (int j8 = 0; j8 < 32; j8 += 8) {
+        if ((uint32_t)j8 < blocks) {
+#pragma unroll
+          for (int j = j8; j < j8 + 8; ++j) {
+            const int at = (int)kQgram * j, k = at / 32, o = at % 32;
+            const uint32_t x1 = o <= 27 ? b1[k] >> o : __funnelshift_r(b1[k], b1[k + 1], o);
+            const uint32_t x0 = o <= 27 ? b0[k] >> o : __funnelshift_r(b0[k], b0[k + 1], o);
+            hits = 2u * hits + ((set[x1 & 31u] >> (x0 & 31u)) & 1u);
+          }
+        } else {
+          hits <<= 8;
+        }
+      }
+      if (all != 0xFFFFFFFFu) {  // some base outside ACGT (perhaps past the window)
+        uint32_t ok = 0;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          const int at = (int)kQgram * j, k = at / 32, o = at % 32;
+          const uint32_t x = __funnelshift_r(v[k], v[k + 1], o);
+          ok = 2u * ok + ((x & 31u) == 31u ? 1u : 0u);
+        }
+        hits &= ok;
+      }
+      count += (uint32_t)__popc(hits & ~low_mask(32u - blocks));
     }
-#undef KIRA_QG_COUNT
-#undef KIRA_QG_HIT
-    p0 = pw.b0, p1 = pw.b1, pv = pw.v;
-    // Decided once the count reaches a bound or can no longer reach it.
-    const int32_t left = (int32_t)m - (int32_t)(32u * blk + lim);
-    if (count >= hi) return 0u;
-    if (count + left < lo) return 2u;
-    if (count >= lo && count + left < hi) return 1u;
   }
-  return count < lo ? 2u : count < hi ? 1u : 0u;
-}
-#undef KIRA_QG_ALL
-
-// True when the read provably has edit distance > k to every window substring.
-__device__ __forceinline__ bool qgram4_reject(const uint4* __restrict__ rplanes, uint64_t rpos,
-                                              uint32_t m, const uint4* __restrict__ wplanes,
-                                              uint64_t wpos, uint32_t n, uint32_t k,
-                                              uint32_t* set) {
-  const int32_t need = (int32_t)m - 3 - 4 * (int32_t)k;
-  return qgram4_outcome(rplanes, rpos, m, wplanes, wpos, n, need, need, set) != 0u;
+  __syncwarp();  // the sets are free for the next pairs
+  if (!active) return 0u;
+  return (int32_t)count < lo ? 2u : (int32_t)count < hi ? 1u : 0u;
 }
 
 }  // namespace kira
