@@ -2852,14 +2852,29 @@ int kira_gpu_align_batch_simd(kira_ctx* ctx, const kira_pairs* pairs, const kira
     if (group == 16u && !i16_fits(q0, r0, *cfg)) group = 0;  // per-chunk scalar fallback
   }
   if (group == 0) return kira_gpu_bsw_batch(ctx, pairs, cfg, out, cigar, nullptr);
-  // Full-window kernel.
+  // Full-window kernel: packed int16 while the values fit and the trace's H bytes are H
+  // itself (no rescue in this mode), else int32. Eight lanes a pair and more words each do
+  // less work, a warp per pair finishes a row sooner.
   const int cap_need = (int)r0;
+  const SwParams fsp = resolve(*cfg);
   int shape = -1;
-  for (int s = 0; s < kNumBswShapes; ++s)
-    if (!kBswShapes[s].packed && shape_cap(kBswShapes[s]) >= cap_need) {
-      shape = s;
-      break;
-    }
+  if (!packed_trace_wraps(q0, fsp)) {
+    constexpr int kMany[] = {10, 11, 26, 27}, kFew[] = {24, 25, 13};
+    constexpr uint32_t kManyPairs = 1500;
+    for (int s : kMany)
+      if (n >= kManyPairs && shape < 0 && shape_cap(kBswShapes[s]) >= cap_need &&
+          packed_fits(kBswShapes[s], q0, fsp))
+        shape = s;
+    for (int s : kFew)
+      if (shape < 0 && shape_cap(kBswShapes[s]) >= cap_need &&
+          packed_fits(kBswShapes[s], q0, fsp))
+        shape = s;
+  }
+  // (Windows up to 544, the widest int32 row, whichever kernel runs.)
+  int wide = -1;
+  for (int s = 0; s < kNumBswShapes && wide < 0; ++s)
+    if (!kBswShapes[s].packed && shape_cap(kBswShapes[s]) >= cap_need) wide = s;
+  if (shape < 0 || wide < 0) shape = wide;
   if (shape < 0)
     return fail(ctx, KIRA_ERR_INVALID, "full-window batch: window of %u > supported 544", r0);
   if (cfg->gap_open < 0 || cfg->gap_extend < 0)
@@ -2886,7 +2901,8 @@ int kira_gpu_align_batch_simd(kira_ctx* ctx, const kira_pairs* pairs, const kira
   if (P.abort_score)
     for (uint32_t i = 0; i < n && !any_abort; ++i) any_abort = P.abort_score[i] > kAbortOff;
   B.count = n;
-  B.sp = resolve(*cfg);
+  B.sp = fsp;
+  B.bias = packed_bias(kBswShapes[shape], fsp);
   B.out = dout;
   B.ncig = ncig;
   B.flags = counters + 2;

@@ -134,7 +134,7 @@ __device__ __forceinline__ uint32_t bsw16_onehot4(uint32_t w) {
 // lies past the one holding the window's last byte `last`, so bytes past the window
 // end are whatever that word holds (those cells are never active). Short lanes: the
 // bytes; long ones: one-hot classes (`raw` < 0), or 0x80 where the byte equals `raw`.
-template <int K>
+template <int K, bool CLASSES = (K >= 17)>
 __device__ __forceinline__ void bsw16_window_words(uint32_t (&wb)[(K + 1) / 2],
                                                    const uint8_t* a, const uint8_t* b,
                                                    const uint8_t* last, int32_t raw) {
@@ -149,7 +149,7 @@ __device__ __forceinline__ void bsw16_window_words(uint32_t (&wb)[(K + 1) / 2],
     return __ldg(reinterpret_cast<const uint32_t*>(x < la ? x : la));
   };
   auto enc = [raw, q4](uint32_t w) {
-    if constexpr (K < 17) return w;
+    if constexpr (!CLASSES) return w;
     const uint32_t t = w ^ q4;
     return raw < 0 ? bsw16_onehot4(w)
                    : ~(((t & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | t) & 0x80808080u;
@@ -689,6 +689,147 @@ __device__ __forceinline__ void bsw16_group_sweep(
   out.end_j = bj;
   out.early_abort = early;
   cells_out = cells;
+}
+
+// The packed full-window sweep of align_batch_simd (sw_batch_avx2_inner,
+// src/alignment/mod.rs:1914-2135): every row covers columns 1 .. w, no band, no x-drop;
+// same layout and trace as the banded sweep (row start 1, row length w). The row is
+// bound by the latency and issue of its few words: the window stays in registers for
+// the whole read, the diagonal predecessor is the word before, nothing moves.
+//   Cells past the window (c >= w) never reach a cell inside it, and with their diagonal
+// held at 0 their H never passes column w's (E and F decay from it alone), so a row's
+// first maximum needs no mask. `rowkeys`: per-row keys for the group abort rule (null:
+// no bound is active).
+template <int G, int K>
+__device__ __forceinline__ void bsw16_full_sweep(
+    const uint8_t* __restrict__ rd, uint32_t q, const uint8_t* __restrict__ wn, uint32_t w,
+    const SwParams& sp, int32_t bias, uint8_t* __restrict__ trace, uint32_t* __restrict__ meta,
+    uint32_t g, uint32_t gmask, DpEnd& out, uint32_t* __restrict__ rowkeys) {
+  constexpr int H = G * K;
+  constexpr int NW = (K + 1) / 2;
+  constexpr int NS = Bsw16Shape<G, K>::kSlabs;
+  constexpr int R = Bsw16Shape<G, K>::kInterleave;
+  constexpr int KB = Bsw16Shape<G, K>::kKeyBits;
+  constexpr uint32_t KM = (1u << KB) - 1u;
+  static_assert(G >= 8, "groups that store whole sectors");
+  const int32_t gi = (int32_t)g, c0 = gi * K;
+  const int32_t gof = sp.gof, ge = sp.gap_extend;
+  const uint32_t B2 = pk2(bias), BG2 = pk2(bias - gof);
+  const uint32_t MAT2 = pk2(sp.match + gof), MIS2 = pk2(gof - sp.mismatch), NGE2 = pk2(-ge);
+  const uint32_t GOFS = isum(gof, gof), NGOF2 = pk2(-gof);
+  const uint32_t GE65537 = (uint32_t)ge * 65537u, DEC0 = ge ? 65536u : 0u;  // pk2(-k * ge)
+  const uint32_t d0 = isum(0x8000 - 1 - c0 + (int32_t)w, 0x8000 - 1 - H - c0 + (int32_t)w);
+  uint32_t ph[K], pe[K], in[K], wb[NW];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    ph[k] = BG2;
+    pe[k] = 0u;
+    in[k] = bsw16_act(d0, k);  // the cells inside the window
+  }
+  if (w) bsw16_window_words<K, false>(wb, wn + c0, wn + H + c0, wn + (w - 1), -1);
+  int32_t best = 0, bi = 0, bj = 0, bq = 0, bqj = 0;
+  uint32_t qb_next = q ? ldb(rd, 0) : 0u;
+  for (uint32_t iu = 1; iu <= q; ++iu) {
+    const int32_t i = (int32_t)iu;
+    if (w == 0) {  // mod.rs:1437-1444
+      if (g == 0) {
+        meta[i] = (1u << 11);
+        if (rowkeys) rowkeys[i] = 0;
+      }
+      continue;
+    }
+    const uint32_t qb4 = qb_next * 0x01010101u;
+    if (iu < q) qb_next = ldb(rd, (uint64_t)iu);
+    // The diagonal predecessor of a lane's first word: the previous lane's last word
+    // (lane 0: column 0, H = 0, in the low half; cell H - 1 in the high half).
+    uint32_t diag = __shfl_sync(gmask, ph[K - 1], (gi + G - 1) & (G - 1), G);
+    if (gi == 0) diag = prmt(BG2, diag, 0x5410u);
+    uint32_t z = 0u, f = 0u;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      if ((k & 1) == 0) {  // top bit of each byte: different
+        const uint32_t x = wb[k >> 1] ^ qb4;
+        z = x | ((x & 0x7F7F7F7Fu) + 0x7F7F7F7Fu);
+      }
+      const uint32_t uh = ph[k];
+      const uint32_t e = __viaddmax_s16x2(pe[k], NGE2, uh);  // max(E_up - ge, H_up - gof)
+      const uint32_t ms = prmt(z, 0u, (k & 1) ? 0xBBAAu : 0x9988u);
+      const uint32_t hm = bsel(B2, __viaddmax_s16x2(diag, bsel(MAT2, MIS2, ms), B2), in[k]);
+      const uint32_t tg = __vimax_s16x2_relu(hm, e) - GOFS;
+      ph[k] = __viaddmax_s16x2(f, NGOF2, tg);  // H - gof
+      f = __viaddmax_s16x2(f, NGE2, tg);
+      pe[k] = e;
+      diag = uh;
+    }
+    uint32_t v = f;
+#pragma unroll
+    for (int off = 1; off < G; off <<= 1) {
+      const uint32_t tt = __shfl_up_sync(gmask, v, off, G);
+      if (gi >= off) v = __viaddmax_s16x2(tt, pk2(-off * K * ge), v);
+    }
+    uint32_t excl = __shfl_up_sync(gmask, v, 1, G);
+    if (gi == 0) excl = 0u;
+    const uint32_t tot = __shfl_sync(gmask, v, G - 1, G);
+    excl = __viaddmax_s16x2(prmt(tot, 0u, 0x1054u), pk2(-c0 * ge) & 0xFFFF0000u, excl);
+    excl = __viaddmax_s16x2(excl, NGOF2, 0u);
+    uint32_t mx = 0u, mx1 = 0u, ka = 0u;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      uint32_t dec = 0u;
+      if (k) asm volatile("mad.lo.u32 %0, %1, %2, %3;" : "=r"(dec) : "r"(GE65537), "r"(-k), "r"(DEC0));
+      ph[k] = __viaddmax_s16x2(excl, dec, ph[k]);
+      const uint32_t kk = ph[k] * (1u << KB) + (KM - (uint32_t)k) * 0x10001u;
+      if (k & 1) {
+        if (k & 2) mx1 = __vimax3_u16x2(mx1, ka, kk);
+        else mx = __vimax3_u16x2(mx, ka, kk);
+      }
+      ka = kk;
+    }
+    if (K & 1) mx = __vimax3_u16x2(mx, ka, 0u);
+    mx = __vimax3_u16x2(mx, mx1, 0u);
+    uint32_t* trow = reinterpret_cast<uint32_t*>(
+                         trace + (size_t)(i / R) * Bsw16Shape<G, K>::kStripBytes) +
+                     (i & (R - 1)) * G + g;
+#pragma unroll
+    for (int x = 0; x < NS; ++x)
+      trow[x * R * G] = prmt(ph[2 * x], 2 * x + 1 < K ? ph[2 * x + 1 < K ? 2 * x + 1 : 0] : 0u,
+                             0x6420u);
+    const uint32_t vlo = (mx & 0xFFFFu) >> KB, vhi = mx >> (16 + KB);
+    const bool lo_first = vlo >= vhi;
+    const uint32_t idx = lo_first ? (uint32_t)c0 + (KM - (mx & KM))
+                                  : (uint32_t)(H + c0) + (KM - ((mx >> 16) & KM));
+    uint32_t key = ((lo_first ? vlo : vhi) << 11) | (2047u - idx);
+    if constexpr (G == 32) {
+      key = __reduce_max_sync(gmask, key);
+    } else {
+#pragma unroll
+      for (int off = G / 2; off > 0; off >>= 1) key = max(key, __shfl_xor_sync(gmask, key, off, G));
+    }
+    const int32_t row_best = (int32_t)(key >> 11) - (bias - gof);
+    const int32_t j = 1 + (2047 - (int32_t)(key & 2047u));
+    if (g == 0) {
+      meta[i] = (1u << 11) | w;
+      if (rowkeys) rowkeys[i] = ((uint32_t)row_best << kKeyIdxBits) | (uint32_t)(1023 - (j - 1));
+    }
+    if (row_best > best) {
+      best = row_best;
+      bi = i;
+      bj = j;
+    }
+    if (iu == q && row_best > bq) {
+      bq = row_best;
+      bqj = j;
+    }
+  }
+  if (bq > 0 && sat_add(bq, sp.clip) > best) {
+    best = bq;
+    bi = (int32_t)q;
+    bj = bqj;
+  }
+  out.score = best;
+  out.end_i = bi;
+  out.end_j = bj;
+  out.early_abort = 0;
 }
 
 // Trace bytes of the packed sweep: hb(i, j) is the low byte of H of cell (i, j), or -1

@@ -593,6 +593,29 @@ __global__ void __launch_bounds__(T, MINB) bsw16_dp_kernel(DevPairs P, BswLaunch
   if (g == 0) bulk_copies_done();  // the trace copies this lane issued
 }
 
+// Packed full-window sweep (bsw16_full_sweep): a group per item, in input order.
+template <int G, int K>
+__global__ void __launch_bounds__(32, 16) bsw16_full_kernel(DevPairs P, BswLaunch B) {
+  const uint32_t g = threadIdx.x % G, gw = threadIdx.x / G;
+  const uint32_t gmask = (G == 32) ? 0xFFFFFFFFu : (((1u << G) - 1u) << (gw * G));
+  for (uint32_t item = blockIdx.x * (32u / G) + gw; item < B.count; item += gridDim.x * (32u / G)) {
+    const uint32_t q = P.read_len[item], w = P.win_len[item];
+    if (q > B.max_q || w > 2u * G * K) {  // outside the shape
+      if (g == 0) {
+        B.ends[item] = DpEnd{0, 0, 0, kEndOutsideShape};
+        atomicOr(B.flags, 2u);
+      }
+      continue;
+    }
+    DpEnd end;
+    bsw16_full_sweep<G, K>(P.read_seq + P.read_off[item], q, P.win_seq + P.win_off[item], w, B.sp,
+                           B.bias, B.tg.trace + (size_t)item * B.tg.slot_bytes,
+                           B.tg.meta + (size_t)item * B.tg.meta_stride, g, gmask, end,
+                           B.rowkeys ? B.rowkeys + (size_t)item * B.tg.meta_stride : nullptr);
+    if (g == 0) B.ends[item] = end;
+  }
+}
+
 // An item's result row, from its end and where its walk stopped (i, j).
 __device__ __forceinline__ void write_sw_row(const BswLaunch& B, uint32_t item, uint32_t pair,
                                              const DpEnd& e, bool outside, int32_t i, int32_t j,
@@ -967,6 +990,15 @@ cudaError_t launch_myers(const DevPairs& P, const MyersLaunch& M, uint32_t max_i
   return cudaGetLastError();
 }
 
+// The group abort rule of the full-window mode over the sweep's row keys.
+static cudaError_t launch_full_abort(const DevPairs& P, const BswLaunch& B, cudaStream_t st) {
+  if (!B.rowkeys) return cudaSuccess;
+  const int rb = (int)((B.count + 127) / 128);
+  (bsw_full_done_kernel<<<rb, 128, 0, st>>>(P, B), count_launch());
+  (bsw_full_resolve_kernel<<<rb, 128, 0, st>>>(P, B), count_launch());
+  return cudaGetLastError();
+}
+
 template <int G, int K, int T, int MINB>
 static cudaError_t launch_bsw_shape(const DevPairs& P, const BswLaunch& B, uint32_t max_items,
                                     int sms, cudaStream_t st, cudaEvent_t between, int parts) {
@@ -983,11 +1015,8 @@ static cudaError_t launch_bsw_shape(const DevPairs& P, const BswLaunch& B, uint3
     (kern<<<blocks, threads, smem, st>>>(P, B), count_launch());
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    if (B.full && B.rowkeys) {
-      const int rb = (int)((B.count + 127) / 128);
-      (bsw_full_done_kernel<<<rb, 128, 0, st>>>(P, B), count_launch());
-      (bsw_full_resolve_kernel<<<rb, 128, 0, st>>>(P, B), count_launch());
-      e = cudaGetLastError();
+    if (B.full) {
+      e = launch_full_abort(P, B, st);
       if (e != cudaSuccess) return e;
     }
   }
@@ -1026,6 +1055,18 @@ static cudaError_t launch_bsw16_shape(const DevPairs& P, const BswLaunch& B, uin
   return e;
 }
 
+template <int G, int K>
+static cudaError_t launch_full16(const DevPairs& P, const BswLaunch& B, int sms, cudaStream_t st) {
+  (bsw16_full_kernel<G, K><<<grid_for(B.count, 32 / G, sms * 32), 32, 0, st>>>(P, B),
+   count_launch());
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = launch_full_abort(P, B, st);
+  if (e != cudaSuccess) return e;
+  (bsw_tb_kernel<G, K, true><<<grid_for(B.count, 4, sms * 16), 128, 0, st>>>(P, B),
+   count_launch());
+  return cudaGetLastError();
+}
+
 // Launch shapes (lanes per pair, cells per lane, threads per block, min resident
 // blocks per SM). Installed per band class by the autotuner / override, else picked by
 // default_shape.
@@ -1050,12 +1091,26 @@ const BswShapeInfo kBswShapes[] = {
     // a warp per pair with the fewest words a lane, for the shortest rows: bands up to
     // 63 and 159
     {32, 2, 32, 16, 1},  {32, 5, 32, 16, 1},
+    // full-window batches: windows up to 272 and 544 on 17 words a lane
+    {8, 17, 32, 16, 1},  {16, 17, 32, 16, 1},
 };
 const int kNumBswShapes = 23;
 const int kNumAllBswShapes = sizeof(kBswShapes) / sizeof(kBswShapes[0]);
 
 cudaError_t launch_bsw(int shape, const DevPairs& P, const BswLaunch& B, uint32_t max_items,
                        int sms, cudaStream_t st, cudaEvent_t between, int parts) {
+  if (B.full && kBswShapes[shape].packed) {
+    switch (shape) {
+      case 10: return launch_full16<8, 5>(P, B, sms, st);
+      case 11: return launch_full16<8, 9>(P, B, sms, st);
+      case 26: return launch_full16<8, 17>(P, B, sms, st);
+      case 27: return launch_full16<16, 17>(P, B, sms, st);
+      case 24: return launch_full16<32, 2>(P, B, sms, st);
+      case 25: return launch_full16<32, 5>(P, B, sms, st);
+      case 13: return launch_full16<32, 9>(P, B, sms, st);
+      default: return cudaErrorInvalidValue;
+    }
+  }
   switch (shape) {
 #define KIRA_BSW(S, G, K, T, M) \
   case S: return launch_bsw_shape<G, K, T, M>(P, B, max_items, sms, st, between, parts);
