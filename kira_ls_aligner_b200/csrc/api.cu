@@ -34,7 +34,7 @@ enum BufId {
   B_DIST, B_END, B_SIEVE_OUT, B_SIEVE_JOBS, B_CELLS, B_TOTAL, B_READ_PLANES, B_WIN_PLANES,
   B_ROWKEYS, B_DONE_ROW, B_WORK, B_WFA_MAXS, B_WFA_TBF, B_WFA_OUT, B_WFA_NCIG, B_WFA_SLOTS,
   B_WFA_SCRATCH, B_WFA_FLAGS, B_PF_CHAINS, B_PF_TOP1, B_PF_MARGIN, B_PF_OUT, B_PF_NCIG,
-  B_PF_MDLEN, B_PF_MDOFF, B_PF_MD, B_PF_EXACT, B_WFA_FB, B_WFA_WHIST, B_SIEVE_LIST, B_PACKED, B_STATUS, B_KEEP, B_ROW_OFF,
+  B_PF_MDLEN, B_PF_MDOFF, B_PF_MD, B_PF_EXACT, B_WFA_FB, B_WFA_WHIST, B_WFA_WHIST2, B_SIEVE_LIST, B_PACKED, B_STATUS, B_KEEP, B_ROW_OFF,
   B_ROWS, B_ROW_SUMS, B_ROW_TOTAL, B_SW_GROUPS, B_RESCUE_LIST, B_RESCUE_TRACE, B_RESCUE_META,
   B_COUNT
 };
@@ -149,6 +149,7 @@ struct kira_ctx {
   cudaStream_t cls_st[kBandClasses] = {};
   cudaEvent_t ev_cls_fork = nullptr, ev_cls_join[kBandClasses] = {};
   cudaStream_t h2d = nullptr, d2h = nullptr;   // copy streams of the chunked host path
+  cudaStream_t wfa_tail = nullptr;             // later passes of the chunked WFA
   int64_t chunk_pairs = -1;                    // chunked host path: -1 auto, 0 off, else pairs
   int wfa_lanes = 0;                           // WFA lanes per pair: 0 auto, else 8 / 16 / 32
   std::vector<cudaEvent_t> ev_up, ev_comp;     // per chunk: inputs landed / results ready
@@ -1851,6 +1852,10 @@ void kira_gpu_destroy(kira_ctx* ctx) {
   for (auto e : ctx->ev_scan) cudaEventDestroy(e);
   if (ctx->h2d) cudaStreamDestroy(ctx->h2d);
   if (ctx->d2h) cudaStreamDestroy(ctx->d2h);
+  if (ctx->wfa_tail) {
+    cudaStreamSynchronize(ctx->wfa_tail);
+    cudaStreamDestroy(ctx->wfa_tail);
+  }
   if (ctx->aux) {
     cudaStreamSynchronize(ctx->aux);
     cudaStreamDestroy(ctx->aux);
@@ -2166,11 +2171,11 @@ int kira_gpu_wfa_batch(kira_ctx* ctx, const kira_pairs* pairs, const kira_wfa_pa
   L.slot_cap = (uint32_t)(2 * (S / min_cost) + 2);
   L.max_score_pp = nullptr;
   L.tbf_pp = nullptr;
-  // Fixed-window fast path: 64 diagonals per pair (128 when 64 cover fewer than 32
-  // scores), placed so every cell of the highest score stays inside for this
-  // batch's leading free text; pairs still open at that score fall back to the
-  // general kernel with a warp per pair (their fronts are the wide ones).
-  // ctx->wfa_lanes != 0 forces the general kernel alone.
+  // Fixed-window passes: 64 diagonals per pair, then 128 for what 64 leave open (128
+  // at once when 64 cover fewer than 32 scores), placed so every cell of the highest
+  // score stays inside for this batch's leading free text; pairs still open after
+  // that fall back to the general kernel with a warp per pair (their fronts are the
+  // wide ones). ctx->wfa_lanes != 0 forces the general kernel alone.
   auto place = [&](int width, int* base) {
     int best = -1;
     for (int b = -(width - 1 - (int)tbf_max); b <= 0; ++b) {
@@ -2181,21 +2186,48 @@ int kira_gpu_wfa_batch(kira_ctx* ctx, const kira_pairs* pairs, const kira_wfa_pa
     }
     return best;
   };
-  int win_base = 0, win_segments = 2;
-  int win_smax = tbf_max <= 63 ? place(64, &win_base) : -1;
-  if (win_smax < std::min<int64_t>(S, 32) && tbf_max <= 127) {
-    int b4 = 0;
-    const int s4 = place(128, &b4);
-    if (s4 > win_smax) win_smax = s4, win_base = b4, win_segments = 4;
-  }
-  const bool use_window = ctx->wfa_lanes == 0 && win_smax >= 16 && L.ring_len <= 64;
-  if (use_window) {
-    win_smax = (int)std::min<int64_t>(win_smax, S);
-    L.win_base = win_base;
-    L.win_smax = win_smax;
-    L.win_segments = win_segments;
-    L.win_ring_bytes =
-        (uint32_t)((L.ring_len * 3u * (32u * (uint32_t)win_segments + 2u) * 2u + 15u) & ~15u);
+  WfaWindow win[2] = {};
+  int wins = 0;
+  auto add_window = [&](int width, int base, int smax, int lanes) {
+    WfaWindow& X = win[wins];
+    X.base = base, X.width = width, X.lanes = lanes;
+    X.smax = (int)std::min<int64_t>(smax, S);
+    auto rows = [](int32_t back) {  // the row itself and `back` before it
+      int32_t r = 1;
+      while (r <= back) r *= 2;
+      return r;
+    };
+    X.rows_m = L.lookback + 1, X.rows_i = rows(L.ei), X.rows_d = rows(L.ed);
+    X.ring_bytes =
+        ((uint32_t)(X.rows_m + X.rows_i + X.rows_d + 1) * ((uint32_t)width + 2u) * 2u + 15u) & ~15u;
+    const uint32_t unit = lanes < 32 ? 4u : 1u;  // bytes held per base
+    X.pat_bytes = unit * ((m_max + 15u) & ~15u) + 32u;
+    // 32 bytes past a multiple of 128: the pairs of a warp start on different banks.
+    X.group_bytes = ((X.ring_bytes + X.pat_bytes + unit * ((n_max + 15u) & ~15u) + 96u + 95u) &
+                     ~127u) + 32u;
+    return wfa_window_pairs(X) * X.group_bytes;
+  };
+  if (ctx->wfa_lanes == 0 && R <= 64) {
+    int b64 = 0, b128 = 0;
+    const int s64 = tbf_max <= 63 ? place(64, &b64) : -1;
+    const int s128 = tbf_max <= 127 ? place(128, &b128) : -1;
+    if (s64 >= 16 && s64 >= std::min<int64_t>(S, 32)) {
+      // 16 lanes per pair, two pairs a warp, hide each other's idle lanes (200k pairs of
+      // 100 / 150 / 250 / 400 bases: 0.70 / 1.45 / 3.36 / 8.8 ms against 0.94 / 1.78 /
+      // 3.83 / 9.4 with 32; with 32 free leading bases 2.15 both) while four blocks of
+      // such pairs fit an SM's shared memory; longer reads take a warp each.
+      if (add_window(64, b64, s64, 16) > (56u << 10)) add_window(64, b64, s64, 32);
+      ++wins;
+    }
+    if (s128 >= 16 && (wins ? S > win[0].smax && s128 > s64 : s128 > s64)) {
+      add_window(128, b128, s128, 32);
+      ++wins;
+    } else if (!wins && s64 >= 16) {
+      add_window(64, b64, s64, 32);
+      ++wins;
+    }
+    // Reads too long for a window's shared memory: the general kernel alone.
+    if (wins && wfa_window_pairs(win[wins - 1]) * win[wins - 1].group_bytes > (220u << 10)) wins = 0;
   }
 
   cudaSetDevice(ctx->device);
@@ -2241,32 +2273,41 @@ int kira_gpu_wfa_batch(kira_ctx* ctx, const kira_pairs* pairs, const kira_wfa_pa
                               std::max<uint64_t>(1, kWfaScratchBudget / (gpb * group_bytes)));
   KIRA_DBUF(scratch, uint8_t, B_WFA_SCRATCH, blocks * gpb * group_bytes);
   KIRA_DBUF(dout, kira_wfa_result, B_WFA_OUT, n);
-  KIRA_DBUF(work, uint32_t, B_WORK, 4);  // window fetch, flags, general fetch, fallbacks
+  // Flags, then per chunk the fetch counter of the general kernel and the fetch and the
+  // fallbacks of each window pass.
+  KIRA_DBUF(work, uint32_t, B_WORK, 1 + 5ull * nch);
   KIRA_DBUF(total_dev, uint64_t, B_TOTAL, 1);
   L.scratch = scratch;
-  L.flags = work + 1;
-  uint64_t wblocks = 0;
+  L.flags = work;
+  uint64_t wblocks[2] = {0, 0};
   uint32_t fwpb = 4;
-  if (use_window) {
-    const size_t wsmem = (size_t)4 * (L.win_ring_bytes + L.smem_group - L.ring_bytes);
+  for (int i = 0; i < wins; ++i) {
+    WfaWindow& X = win[i];
+    const uint64_t wpairs = wfa_window_pairs(X);
     int wper = 0;
-    KIRA_CUDA(wfa_window_blocks_per_sm(win_segments, tb, wsmem, &wper));
-    if (wper < 1) return fail(ctx, KIRA_ERR_INVALID, "WFA window: %zu shared bytes", wsmem);
-    wblocks = std::min<uint64_t>((csz + 3) / 4, (uint64_t)ctx->sms * wper);
-    KIRA_DBUF(fb, uint32_t, B_WFA_FB, csz);
-    L.fb_list = fb;
+    KIRA_CUDA(wfa_window_blocks_per_sm(L, X, tb, &wper));
+    if (wper < 1) return fail(ctx, KIRA_ERR_INVALID, "WFA window: %u shared bytes", X.group_bytes);
+    wblocks[i] = std::min<uint64_t>((csz + wpairs - 1) / wpairs, (uint64_t)ctx->sms * wper);
+    const uint64_t block_hist = wpairs * (uint64_t)(X.smax + 1) * (uint64_t)X.width;
+    if (tb) wblocks[i] = std::min(wblocks[i], std::max<uint64_t>(1, kWfaScratchBudget / 4 / block_hist));
+    if (tb && i == 0) {
+      KIRA_DBUF(wh, int32_t, B_WFA_WHIST, wblocks[i] * block_hist);
+      X.hist = wh;
+    } else if (tb) {
+      KIRA_DBUF(wh, int32_t, B_WFA_WHIST2, wblocks[i] * block_hist);
+      X.hist = wh;
+    }
+  }
+  uint32_t* fb = nullptr;
+  if (wins) {
+    KIRA_DBUF(fbl, uint32_t, B_WFA_FB, (uint64_t)wins * n);
+    fb = fbl;
     // Fallback launch shape: 32 lanes per pair, up to 4 warps (pairs) per block; it
     // uses no more groups than the scratch above holds.
     while (fwpb > 1 && (uint64_t)fwpb * L.smem_group > (160u << 10)) fwpb >>= 1;
     int fper = 0;
     KIRA_CUDA(wfa_blocks_per_sm(32, tb, (size_t)fwpb * L.smem_group, (int)(32 * fwpb), &fper));
     if (fper < 1) return fail(ctx, KIRA_ERR_INVALID, "WFA fallback: %u shared bytes", L.smem_group);
-    L.fb_count = work + 3;
-    if (tb) {
-      KIRA_DBUF(wh, int16_t, B_WFA_WHIST,
-                wblocks * 4 * (uint64_t)(win_smax + 1) * 3 * 32 * win_segments);
-      L.win_hist = wh;
-    }
   }
   uint32_t *ncig = nullptr, *off = nullptr, *sums = nullptr, *ops = nullptr;
   if (tb) {
@@ -2278,8 +2319,13 @@ int kira_gpu_wfa_batch(kira_ctx* ctx, const kira_pairs* pairs, const kira_wfa_pa
     ncig = nc, off = of, sums = su, ops = dops;
     L.slots = sl;
   }
-  KIRA_CUDA(cudaMemsetAsync(work, 0, 16, st));
+  KIRA_CUDA(cudaMemsetAsync(work, 0, 4 + 20ull * nch, st));
   KIRA_CUDA(cudaMemsetAsync(total_dev, 0, 8, st));
+  if (chunked && !ctx->wfa_tail) {
+    int least = 0, greatest = 0;
+    KIRA_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    KIRA_CUDA(cudaStreamCreateWithPriority(&ctx->wfa_tail, cudaStreamNonBlocking, greatest));
+  }
   if (chunked) {  // copies start once the buffers exist and the counters are reset
     KIRA_CUDA(cudaEventRecord(ctx->ev_up[nch], st));
     KIRA_CUDA(cudaStreamWaitEvent(ctx->h2d, ctx->ev_up[nch], 0));
@@ -2297,10 +2343,6 @@ int kira_gpu_wfa_batch(kira_ctx* ctx, const kira_pairs* pairs, const kira_wfa_pa
   for (uint32_t c = 0; c < nch; ++c) {
     const uint32_t lo = c * csz, m = std::min(n, lo + csz) - lo;
     if (chunked) KIRA_CUDA(cudaStreamWaitEvent(st, ctx->ev_up[c], 0));
-    if (c) {  // fetch counters of both kernels and the fallback count
-      KIRA_CUDA(cudaMemsetAsync(work, 0, 4, st));
-      KIRA_CUDA(cudaMemsetAsync(work + 2, 0, 8, st));
-    }
     WfaLaunch Lc = L;
     Lc.n = m;
     Lc.out = dout + lo;
@@ -2311,32 +2353,46 @@ int kira_gpu_wfa_batch(kira_ctx* ctx, const kira_pairs* pairs, const kira_wfa_pa
       Lc.slots = L.slots + (size_t)lo * L.slot_cap;
     }
     const DevPairs Dc = chunk_view(D, lo, m);
-    if (use_window) {
-      // Window kernel first; its fallbacks (pairs still open at win_smax) run
-      // through the general kernel over the fallback list.
-      Lc.work = work;
-      KIRA_CUDA(launch_wfa_window(Dc, Lc, (uint32_t)std::min<uint64_t>(wblocks, (m + 3) / 4), tb,
-                                  st));
-      Lc.list = L.fb_list;
-      Lc.list_count = L.fb_count;
+    uint32_t* cw = work + 1 + 5ull * c;
+    Lc.work = cw;
+    cudaStream_t ts = st;
+    for (int i = 0; i < wins; ++i) {
+      WfaWindow& X = win[i];
+      X.work = cw + 1 + 2 * i;
+      X.fb_count = cw + 2 + 2 * i;
+      X.fb_list = fb + (size_t)i * n + lo;
+      X.list = i ? win[i - 1].fb_list : nullptr;
+      X.list_count = i ? win[i - 1].fb_count : nullptr;
+      const uint32_t wpairs = wfa_window_pairs(X);
+      KIRA_CUDA(launch_wfa_window(
+          Dc, Lc, X, (uint32_t)std::min<uint64_t>(wblocks[i], (m + wpairs - 1) / wpairs), tb, ts));
+      if (i == 0 && chunked) {
+        // What the first pass leaves open is a few pairs with long serial searches: they
+        // and the chunk's scan run beside the next chunk's first pass.
+        KIRA_CUDA(cudaEventRecord(ctx->ev_pack[c], st));
+        KIRA_CUDA(cudaStreamWaitEvent(ctx->wfa_tail, ctx->ev_pack[c], 0));
+        ts = ctx->wfa_tail;
+      }
+    }
+    if (wins && S > win[wins - 1].smax) {
+      Lc.list = win[wins - 1].fb_list;
+      Lc.list_count = win[wins - 1].fb_count;
       Lc.group = 32;
-      Lc.work = work + 2;
       KIRA_CUDA(launch_wfa(Dc, Lc,
                            (uint32_t)std::max<uint64_t>(
                                1, std::min<uint64_t>(blocks * gpb / fwpb, (m + fwpb - 1) / fwpb)),
-                           fwpb, tb, st));
-    } else {
-      Lc.work = work + 2;
+                           fwpb, tb, ts));
+    } else if (!wins) {
       const uint32_t bl = (uint32_t)std::min<uint64_t>(blocks, (m + gpb - 1) / gpb);
-      KIRA_CUDA(launch_wfa(Dc, Lc, bl, wpb, tb, st));
+      KIRA_CUDA(launch_wfa(Dc, Lc, bl, wpb, tb, ts));
     }
     mark(ctx, 2, st);
     if (tb) {
-      KIRA_CUDA(launch_cigar_scan(ncig + lo, m, off + lo, sums, total_dev, st, true));
+      KIRA_CUDA(launch_cigar_scan(ncig + lo, m, off + lo, sums, total_dev, ts, true));
       WfaCompact C{m, dout + lo, ncig + lo, off + lo, Lc.slots, L.slot_cap, ops, cigar->cap};
-      KIRA_CUDA(launch_wfa_compact(C, ctx->sms, st));
+      KIRA_CUDA(launch_wfa_compact(C, ctx->sms, ts));
     }
-    if (chunked) KIRA_CUDA(cudaEventRecord(ctx->ev_comp[c], st));
+    if (chunked) KIRA_CUDA(cudaEventRecord(ctx->ev_comp[c], ts));
   }
   for (uint32_t c = 0; chunked && c < nch; ++c) {
     const uint32_t lo = c * csz, m = std::min(n, lo + csz) - lo;
@@ -2348,7 +2404,7 @@ int kira_gpu_wfa_batch(kira_ctx* ctx, const kira_pairs* pairs, const kira_wfa_pa
   cudaStream_t dn = chunked ? ctx->d2h : st;
   uint64_t total = 0;
   uint32_t flags = 0;
-  KIRA_CUDA(cudaMemcpyAsync(&flags, work + 1, 4, cudaMemcpyDeviceToHost, dn));
+  KIRA_CUDA(cudaMemcpyAsync(&flags, work, 4, cudaMemcpyDeviceToHost, dn));
   if (tb) KIRA_CUDA(cudaMemcpyAsync(&total, total_dev, 8, cudaMemcpyDeviceToHost, dn));
   if (!chunked)
     KIRA_CUDA(cudaMemcpyAsync(out, dout, sizeof(kira_wfa_result) * n, cudaMemcpyDeviceToHost, dn));

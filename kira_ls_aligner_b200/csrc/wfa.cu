@@ -26,8 +26,7 @@ __device__ __forceinline__ int wfa_high_bit(unsigned b) { return 31 - __clz(b); 
 // the diagonal at termination (the alignment's text start). get(layer, score, k)
 // returns the stored offset or kWfaNone.
 template <class Get>
-__device__ int wfa_traceback_t(const WfaLaunch& L, Get get, const uint32_t* pw,
-                               const uint32_t* tw, int m, int n, int s, int k,
+__device__ int wfa_traceback_t(const WfaLaunch& L, Get get, int m, int n, int s, int k,
                                uint32_t* __restrict__ slot, uint32_t& nops, bool& overflow) {
   uint32_t last = 0xFFFFFFFFu;  // op of the newest entry
   auto push = [&](uint32_t op, uint32_t len) {
@@ -47,13 +46,14 @@ __device__ int wfa_traceback_t(const WfaLaunch& L, Get get, const uint32_t* pw,
     if (layer == 0) {
       const int iv = get(1, s, k), dv = get(2, s, k);
       const int pv = s >= x ? get(0, s - x, k) : kWfaNone;
-      // The walk stops at the first landing point of an edge at or below off.
+      // off is M[s][k] after its extension and the highest edge its value before, so
+      // the bases between are equal: the walk (wfa.rs:807-853) down to the first landing
+      // point of an edge at or below off needs no comparison.
       int low = max(0, -k);
       if (iv != kWfaNone && iv <= off) low = max(low, iv);
       if (dv != kWfaNone && dv <= off) low = max(low, dv);
       if (pv != kWfaNone && pv + 1 <= off) low = max(low, pv + 1);
-      const int run = (off > low && off - 1 < m && off - 1 + k < n) ? wfa_back_run(pw, tw, k, off, low)
-                                                                    : 0;
+      const int run = off > low ? off - low : 0;
       if (run > 0) push(0u, (uint32_t)run);
       off -= run;
       if (s == 0 && off == 0) break;
@@ -102,14 +102,13 @@ __device__ int wfa_traceback_t(const WfaLaunch& L, Get get, const uint32_t* pw,
 }
 
 __device__ int wfa_traceback(const WfaLaunch& L, const int2* __restrict__ meta,
-                             const int16_t* __restrict__ H, const uint32_t* pw,
-                             const uint32_t* tw, int m, int n, int s, int k,
+                             const int16_t* __restrict__ H, int m, int n, int s, int k,
                              uint32_t* __restrict__ slot, uint32_t& nops, bool& overflow) {
   auto get = [&](int layer, int sc, int kk) -> int {
     if (sc < 0) return kWfaNone;
     return wfa_get(H, wfa_unpack(meta[(uint32_t)sc * 3u + layer]), kk);
   };
-  return wfa_traceback_t(L, get, pw, tw, m, n, s, k, slot, nops, overflow);
+  return wfa_traceback_t(L, get, m, n, s, k, slot, nops, overflow);
 }
 
 // G lanes align one pair; the 32 / G groups of a warp step in lockstep through
@@ -365,7 +364,7 @@ __global__ void __launch_bounds__(128) wfa_kernel(DevPairs P, WfaLaunch L) {
           if (TB) {
             bool ovf = false;
             uint32_t* slot = L.slots + (size_t)p * L.slot_cap;
-            const int k0 = wfa_traceback(L, meta, H, pw, tw, m, n, s, kdone, slot, nops, ovf);
+            const int k0 = wfa_traceback(L, meta, H, m, n, s, kdone, slot, nops, ovf);
             res.text_start = (uint32_t)max(k0, 0);
             if (ovf) atomicOr(L.flags, 1u);
           }
@@ -379,215 +378,330 @@ __global__ void __launch_bounds__(128) wfa_kernel(DevPairs P, WfaLaunch L) {
   }
 }
 
-// Fixed-window WFA: one warp per pair, lane l owns diagonals win_base + 32 j + l
-// (j < NH) for the whole search. Every cell the recurrence can reach by score
-// win_smax lies in the window (an inserted base moves one diagonal down for at
-// least ei, a deleted base one up for at least ed, the seeds sit on
-// 0..text_begin_free), so up to that score the window is the whole wavefront and
-// no range is tracked; a 32-diagonal segment that no reached diagonal can touch
-// this score (new cells lie within one diagonal of the reached range) stays
-// "none" without being computed. The last lookback + 1 scores live in a shared
-// ring of int16 rows with a guard column on each side (the k - 1 / k + 1
-// neighbours of the edge diagonals read "none"); "none" is any negative value, so
-// the reference's checks become plain max / select: an unreached source stays
-// negative through the +1s of a search. A pair not done by win_smax (and not
-// exhausted) goes to fb_list for the general kernel, which redoes it from scratch.
-template <int NH, bool TB>
-__global__ void __launch_bounds__(128) wfa_window_kernel(DevPairs P, WfaLaunch L) {
-  constexpr int kW = 32 * NH;  // diagonals of the window
-  constexpr int kRow = kW + 2; // + 2 guards
+// Bytes [0, len) of src to shared memory by the G lanes of a group, a word per lane
+// at a time; reads only aligned words that hold one of the bytes. WIDE: word i of dst
+// holds bytes i .. i + 3, so four bytes from any offset are one load.
+template <int G, bool WIDE>
+__device__ __forceinline__ void wfa_stage(uint32_t* dst, const uint8_t* src, int len, int gl) {
+  const int a = (int)((uintptr_t)src & 3u);
+  const uint32_t* w = (const uint32_t*)(src - a);
+  const uint32_t sel = 0x3210u + 0x1111u * (uint32_t)a;
+  for (int i = gl; 4 * i < len; i += G) {
+    const uint32_t lo = __ldg(w + i);
+    const uint32_t hi = 4 * (i + 1) < a + len ? __ldg(w + i + 1) : 0u;
+    const uint32_t v = __byte_perm(lo, hi, sel);
+    if (WIDE) {
+      const uint32_t nx = __byte_perm(hi, 4 * (i + 2) < a + len ? __ldg(w + i + 2) : 0u, sel);
+      ((uint4*)dst)[i] = make_uint4(v, __byte_perm(v, nx, 0x4321u), __byte_perm(v, nx, 0x5432u),
+                                    __byte_perm(v, nx, 0x6543u));
+    } else {
+      dst[i] = v;
+    }
+  }
+}
+
+// wfa_extend over WIDE arrays (0 <= v <= m, 0 <= v + k <= n).
+__device__ __forceinline__ int wfa_extend_wide(const uint32_t* pe, const uint32_t* te, int m,
+                                               int n, int k, int v) {
+  const uint32_t* a = pe + v;
+  const uint32_t* b = te + v + k;
+  const int lim = min(m - v, n - k - v);
+  uint32_t d = a[0] ^ b[0];
+  int run = 0;
+  if (d == 0) {  // one diagonal of 256 off the alignment's path; 16 bytes a turn on it
+    run = 4;
+    while (run < lim) {
+      const uint32_t d0 = a[run] ^ b[run], d1 = a[run + 4] ^ b[run + 4];
+      const uint32_t d2 = a[run + 8] ^ b[run + 8], d3 = a[run + 12] ^ b[run + 12];
+      if (d0 | d1 | d2 | d3) {
+        if (!(d0 | d1)) run += 8;
+        const uint32_t e0 = d0 | d1 ? d0 : d2, e1 = d0 | d1 ? d1 : d3;
+        if (!e0) run += 4;
+        d = e0 ? e0 : e1;
+        break;
+      }
+      run += 16;
+    }
+  }
+  if (d) run += (__ffs(d) - 1) >> 3;
+  return v + min(run, lim);
+}
+
+// A reached cell of the window kernel's history: M before its extension (from bit 4),
+// whether that came from I or D (else from M at a mismatch), and whether the cell's I
+// and D opened there.
+constexpr int kFromI = 1, kFromD = 2, kIOpen = 4, kDOpen = 8;
+
+// Traceback over those cells in one lane: the edge order of wfa_traceback_t (mismatch,
+// I, D; open before extend) was applied when the cell was computed, so a step is one
+// load. hist is indexed by s * W + k.
+__device__ int wfa_window_traceback(const WfaLaunch& L, const int* hist, int W, int m, int s,
+                                    int k, uint32_t* __restrict__ slot, uint32_t& nops,
+                                    bool& overflow) {
+  uint32_t op = 0, len = 0;
+  auto push = [&](uint32_t o, uint32_t l) {
+    if (o != op) {
+      if (len) {
+        if (nops < L.slot_cap) slot[nops] = len << 4 | op;
+        else overflow = true;
+        ++nops;
+      }
+      op = o, len = 0;
+    }
+    len += l;
+  };
+  int off = m, layer = 0;
+  while (s > 0) {
+    const int c = hist[s * W + k];
+    if (layer == 0) {
+      const int pre = c >> 4;
+      if (off > pre) push(0u, (uint32_t)(off - pre));
+      off = pre;
+      layer = c & 3;
+      if (layer == 0) {
+        push(0u, 1u);
+        off -= 1, s -= L.x;
+        continue;
+      }
+    }
+    if (layer == kFromI) {
+      push(1u, 1u);
+      off -= 1, k += 1;
+      layer = c & kIOpen ? 0 : kFromI;
+      s -= L.ei + (layer ? 0 : L.o);
+    } else {
+      push(2u, 1u);
+      k -= 1;
+      layer = c & kDOpen ? 0 : kFromD;
+      s -= L.ed + (layer ? 0 : L.o);
+    }
+  }
+  if (off > 0) push(0u, (uint32_t)off);
+  push(~0u, 0u);
+  return k;
+}
+
+// Fixed-window WFA: G lanes per pair, the 32 / G pairs of a warp in lockstep over
+// their rows (scores). Every cell the recurrence can reach by score smax lies in the
+// window's `width` diagonals from `base` (an inserted base moves one diagonal down for
+// at least ei, a deleted base one up for at least ed, the seeds sit on
+// 0..text_begin_free); by score s that is lo = -(s - o) / ei to
+// hi = text_begin_free + (s - o) / ed, taken G diagonals at a time from lo. Each layer
+// keeps as many rows as the recurrence looks back in it, in a shared ring of int16
+// with a guard column on each side; "none" is any negative value, so the reference's
+// checks become plain max / select: an unreached source stays negative through the
+// +1s of a search. A row's range only grows, so a slot never holds an older value
+// outside it. Rows whose sources are all dead (scores 1-4 and 6 at mismatch 5, gaps 7
+// and 8) are passed over: a bit per row tells which hold a value, and a dead source
+// reads a row of "none". A group whose pair is done takes the next one when kWait
+// groups are: a pair's cells grow with the square of its score, so a warp that waits
+// for all its pairs idles most of its lanes. A pair not done by smax (and not
+// exhausted) goes to fb_list.
+//
+// Bound by the instructions issued, 80 % of the slots: 1M pairs of 150 bases at 0-4 %
+// error (265 cells a pair on average) 5.5 ms with the later passes, where a warp per
+// pair over the whole window, with the offsets of every row kept for a traceback that
+// compared bases again, took 8.7.
+template <int G, bool TB, class Mask>
+__global__ void __launch_bounds__(128) wfa_window_kernel(DevPairs P, WfaLaunch L, WfaWindow X) {
+  constexpr int NG = 32 / G;
+  constexpr bool kWide = G < 32;
+  constexpr int kWait = (NG + 1) / 2;
   constexpr int kNone16 = -32000;
   extern __shared__ __align__(16) uint8_t wfa_smem[];
   const int lane = threadIdx.x & 31;
+  const int g = lane / G, gl = lane % G, gbase = g * G;
+  const unsigned gmask = (kFull >> (32 - G)) << gbase;
   const uint32_t wib = threadIdx.x >> 5;
-  const uint32_t stage = L.smem_group - L.ring_bytes;  // pattern + text bytes per warp
-  uint8_t* my = wfa_smem + (size_t)wib * (L.win_ring_bytes + stage);
-  int16_t* ring = (int16_t*)my;
-  uint32_t* pw = (uint32_t*)(my + L.win_ring_bytes + 16);
-  uint32_t* tw = (uint32_t*)(my + L.win_ring_bytes + L.pat_region + 16);
-  uint8_t* pb = (uint8_t*)pw;
-  uint8_t* tb = (uint8_t*)tw;
-  const uint32_t warp = blockIdx.x * (blockDim.x >> 5) + wib;
-  int16_t* hist = TB ? L.win_hist + (size_t)warp * (L.win_smax + 1) * 3 * kW : nullptr;
-  const int R = (int)L.ring_len;
+  const int W = X.width, rowlen = W + 2, base = X.base;
+  uint8_t* my = wfa_smem + (size_t)(wib * NG + (uint32_t)g) * X.group_bytes;
+  uint32_t* pw = (uint32_t*)(my + X.ring_bytes + 16);
+  uint32_t* tw = (uint32_t*)(my + X.ring_bytes + X.pat_bytes + 16);
   const int x = L.x, oi = L.o + L.ei, od = L.o + L.ed, ei = L.ei, ed = L.ed;
-  const int xr = x % R, oir = oi % R, odr = od % R, eir = ei % R, edr = ed % R;
-  const int base = L.win_base;
-  for (int r = lane; r < R * 3; r += 32) {  // guard columns stay "none"
-    ring[r * kRow] = (int16_t)kNone16;
-    ring[r * kRow + kRow - 1] = (int16_t)kNone16;
-  }
+  const int rm = X.rows_m;                          // rows of M's ring
+  const int ri = X.rows_i - 1, rd = X.rows_d - 1;  // of I's and D's - 1 (powers of two)
+  int16_t* ringM = (int16_t*)my + 1 - base;
+  int16_t* none_row = ringM + X.rows_m * rowlen;  // what a dead source reads
+  int16_t* ringI = none_row + rowlen;
+  int16_t* ringD = ringI + X.rows_i * rowlen;
+  const uint32_t grp = (blockIdx.x * (blockDim.x >> 5) + wib) * NG + (uint32_t)g;
+  int* hist = TB ? X.hist + (size_t)grp * (X.smax + 1) * W : nullptr;
+  const Mask one = 1;
+  const Mask bx = one << (x - 1), boi = one << (oi - 1), bod = one << (od - 1);
+  const Mask bei = one << (ei - 1), bed = one << (ed - 1);
+  const Mask in_ring = (one << L.lookback << 1) - one;
+  const uint32_t count = X.list ? *X.list_count : L.n;
+
+  bool alive = false, mine = false, dead = false, more = true;
+  uint32_t p = 0;
+  int m = 0, n = 0, S_loop = 0, s_lim = 0, tbf = 0;
+  int s = 0, sm = 0, lo = 0, hi = 0, ci = 0, cd = 0;
+  int done_s = -1, k_end = 0;
+  Mask live_m = 0, live_g = 0;  // bit j: row s - 1 - j holds a value (in I or D)
+  auto advance = [&]() {
+    ++s;
+    if (++sm == rm) sm = 0;
+    if (++ci == ei) ci = 0, --lo;
+    if (++cd == ed) cd = 0, ++hi;
+  };
   for (;;) {
-    uint32_t p = 0;
-    if (lane == 0) p = atomicAdd(L.work, 1u);
-    p = __shfl_sync(kFull, p, 0);
-    if (p >= L.n) break;
-    const int m = (int)P.read_len[p], n = (int)P.win_len[p];
-    if (!L.valid || m == 0) {  // WfaCosts::scored refused: None; empty read: wfa.rs:555-563
-      if (lane == 0) {
-        kira_wfa_result res{};
-        res.cost = L.valid ? 0 : -1;
-        res.found = L.valid ? 1u : 0u;
-        L.out[p] = res;
-        if (TB) L.ncig[p] = 0;
-      }
-      continue;
-    }
-    const uint8_t* rs = P.read_seq + P.read_off[p];
-    const uint8_t* ws = P.win_seq + P.win_off[p];
-    __syncwarp();
-    for (int i = lane; i < m; i += 32) pb[i] = __ldg(rs + i);
-    for (int i = lane; i < n; i += 32) tb[i] = __ldg(ws + i);
-    int S = L.max_score_pp ? L.max_score_pp[p] : L.max_score;
-    if (!L.max_score_pp && S < 0) S = wfa_budget(m, L);
-    const int64_t cap = L.drop < 0 ? (int64_t)L.o + (int64_t)L.ei * m
-                                   : (int64_t)max(x, oi) * (2 * m + n + 2);
-    const int S_loop = (int)max((int64_t)0, min((int64_t)S, cap));
-    const int s_lim = min(S_loop, L.win_smax);
-    int tbf = L.tbf_pp ? L.tbf_pp[p] : L.tbf;
-    tbf = min(max(tbf, 0), max(n - 1, 0));
-    __syncwarp();
-    int done_s = -1, k_end = 0, last_live = 0, slot = 0;
-    int lo_seen = 0, hi_seen = tbf;  // reached diagonals so far (the seeds: 0 .. tbf)
-    bool dead = false;
-    for (int s = 0; s <= s_lim; ++s) {
-      bool need[NH];
-#pragma unroll
-      for (int h = 0; h < NH; ++h)
-        need[h] = lo_seen - 1 <= base + 32 * h + 31 && hi_seen + 1 >= base + 32 * h;
-      auto row = [&](int back, int backr, int layer) -> const int16_t* {
-        int sl = slot - backr;
-        if (sl < 0) sl += R;
-        return (s - back >= 0) ? ring + (sl * 3 + layer) * kRow : nullptr;
-      };
-      const int16_t* rMx = row(x, xr, 0);
-      const int16_t* rMoi = row(oi, oir, 0);
-      const int16_t* rMod = row(od, odr, 0);
-      const int16_t* rIe = row(ei, eir, 1);
-      const int16_t* rDe = row(ed, edr, 2);
-      int16_t* wM = ring + (slot * 3 + 0) * kRow;
-      int16_t* wI = ring + (slot * 3 + 1) * kRow;
-      int16_t* wD = ring + (slot * 3 + 2) * kRow;
-      int vm2[NH], vi2[NH], vd2[NH];
-#pragma unroll
-      for (int h = 0; h < NH; ++h) {
-        const int col = 1 + h * 32 + lane;
-        const int k = base + h * 32 + lane;
-        int vi = kNone16, vd = kNone16, vm = kNone16;
-        if (!need[h]) {
-          // this segment stays "none"
-        } else if (s == 0) {
-          vm = (k >= 0 && k <= tbf) ? 0 : kNone16;
+    const unsigned running = __ballot_sync(kFull, alive);
+    const unsigned waiting = running == kFull ? 0u : __ballot_sync(kFull, !alive && (more || mine));
+    if (!running && !waiting) break;
+    if (!running || __popc(waiting) >= kWait * G) {
+      if (mine && !alive && gl == 0) {  // finish
+        if (done_s < 0 && !dead && S_loop > s_lim) {
+          X.fb_list[atomicAdd(X.fb_count, 1u)] = p;  // redone from scratch
         } else {
-          if (rMoi) {
-            const int a = rMoi[col + 1];
-            vi = a < m ? a + 1 : kNone16;
+          kira_wfa_result res{};
+          res.cost = -1;
+          uint32_t nops = 0;
+          if (done_s >= 0) {
+            res.found = 1;
+            res.cost = done_s;
+            res.score = L.scored ? m * L.match - done_s : done_s;
+            res.text_end = (uint32_t)(m + k_end);
+            if (TB) {
+              bool ovf = false;
+              const int k0 = wfa_window_traceback(L, hist - base, W, m, done_s, k_end,
+                                                  L.slots + (size_t)p * L.slot_cap, nops, ovf);
+              res.text_start = (uint32_t)max(k0, 0);
+              if (ovf) atomicOr(L.flags, 1u);
+            }
           }
-          if (rIe) {
-            const int b = rIe[col + 1];
-            vi = max(vi, b < m ? b + 1 : kNone16);
-          }
-          if (rMod) {
-            const int a = rMod[col - 1];
-            vd = a + k <= n ? a : kNone16;
-          }
-          if (rDe) {
-            const int b = rDe[col - 1];
-            vd = max(vd, b + k <= n ? b : kNone16);
-          }
-          if (rMx) {
-            const int a = rMx[col];
-            vm = (a < m && a + k < n) ? a + 1 : kNone16;
-          }
-          vm = max(vm, max(vi, vd));
-        }
-        if (vm >= 0) vm = wfa_extend(pw, tw, m, n, k, vm);
-        vm2[h] = vm, vi2[h] = vi, vd2[h] = vd;
-      }
-#pragma unroll
-      for (int h = 0; h < NH; ++h) {  // extend the reached range by this score's cells
-        const unsigned q = __ballot_sync(kFull, vm2[h] >= 0 || vi2[h] >= 0 || vd2[h] >= 0);
-        if (q) {
-          lo_seen = min(lo_seen, base + 32 * h + wfa_low_bit(q));
-          hi_seen = max(hi_seen, base + 32 * h + wfa_high_bit(q));
+          if (TB) L.ncig[p] = nops;
+          L.out[p] = res;
         }
       }
-      if (L.drop >= 0) {  // prune_wavefront (wfa.rs:293-346) on the extended M
-        int mad = INT32_MIN;
-#pragma unroll
-        for (int h = 0; h < NH; ++h)
-          if (vm2[h] >= 0) mad = max(mad, 2 * vm2[h] + base + h * 32 + lane);
-        mad = __reduce_max_sync(kFull, mad);
-        if (mad != INT32_MIN) {
-          const int th = mad - L.drop;
-#pragma unroll
-          for (int h = 0; h < NH; ++h)
-            if (vm2[h] >= 0 && 2 * vm2[h] + base + h * 32 + lane < th) vm2[h] = kNone16;
-        }
-      }
-      int kd = INT32_MAX;  // lowest done diagonal
-      bool live = false;
-#pragma unroll
-      for (int h = 0; h < NH; ++h) {
-        const int col = 1 + h * 32 + lane;
-        wM[col] = (int16_t)vm2[h];
-        wI[col] = (int16_t)vi2[h];
-        wD[col] = (int16_t)vd2[h];
-        if (TB) {
-          int16_t* hs = hist + (size_t)s * 3 * kW + h * 32 + lane;
-          hs[0] = (int16_t)vm2[h];
-          hs[kW] = (int16_t)vi2[h];
-          hs[2 * kW] = (int16_t)vd2[h];
-        }
-        const unsigned bd = __ballot_sync(kFull, vm2[h] >= m);
-        if (bd && kd == INT32_MAX) kd = base + 32 * h + wfa_low_bit(bd);
-        live |= (vm2[h] & vi2[h] & vd2[h]) >= 0;  // some value >= 0 unless all negative
-      }
-      live = __any_sync(kFull, live);
       __syncwarp();
+      uint32_t q = 0;
+      if (!alive && more && gl == 0) q = atomicAdd(X.work, 1u);
+      q = __shfl_sync(kFull, q, gbase);
+      if (!alive) {
+        mine = false;
+        more = more && q < count;
+        if (more) {
+          p = X.list ? X.list[q] : q;
+          m = (int)P.read_len[p], n = (int)P.win_len[p];
+          if (!L.valid || m == 0) {  // WfaCosts::scored refused: None; empty read: wfa.rs:555-563
+            if (gl == 0) {
+              kira_wfa_result res{};
+              res.cost = L.valid ? 0 : -1;
+              res.found = L.valid ? 1u : 0u;
+              L.out[p] = res;
+              if (TB) L.ncig[p] = 0;
+            }
+          } else {
+            alive = mine = true;
+            for (uint32_t i = (uint32_t)gl; i < X.ring_bytes / 16u; i += G)
+              ((uint4*)my)[i] = make_uint4(0x83008300u, 0x83008300u, 0x83008300u, 0x83008300u);
+            wfa_stage<G, kWide>(pw, P.read_seq + P.read_off[p], m, gl);
+            wfa_stage<G, kWide>(tw, P.win_seq + P.win_off[p], n, gl);
+            int S = L.max_score_pp ? L.max_score_pp[p] : L.max_score;
+            if (!L.max_score_pp && S < 0) S = wfa_budget(m, L);
+            const int64_t cap = L.drop < 0 ? (int64_t)L.o + (int64_t)L.ei * m
+                                           : (int64_t)max(x, oi) * (2 * m + n + 2);
+            S_loop = (int)max((int64_t)0, min((int64_t)S, cap));
+            s_lim = min(S_loop, X.smax);
+            tbf = L.tbf_pp ? L.tbf_pp[p] : L.tbf;
+            tbf = min(max(tbf, 0), max(n - 1, 0));
+            s = sm = 0;
+            lo = 0, hi = tbf, ci = cd = -L.o;
+            done_s = -1;
+            dead = false;
+            live_m = live_g = 0;
+          }
+        }
+      }
+      __syncwarp();
+      if (!__any_sync(kFull, alive)) continue;
+    }
+
+    // The next row with a live source.
+    if (alive && s > 0) {
+      while (!((live_m & (bx | boi | bod)) | (live_g & (bei | bed)))) {
+        live_m <<= 1, live_g <<= 1;
+        // Nothing reached within the look-back window: no later score reaches anything.
+        dead = (live_m & in_ring) == 0;
+        if (dead || s == s_lim) {
+          alive = false;
+          break;
+        }
+        advance();
+      }
+    }
+    auto back = [&](int b) { return (sm - b + (sm < b ? rm : 0)) * rowlen; };
+    const int16_t* rMx = live_m & bx ? ringM + back(x) : none_row;
+    const int16_t* rMoi = (live_m & boi ? ringM + back(oi) : none_row) + 1;
+    const int16_t* rMod = (live_m & bod ? ringM + back(od) : none_row) - 1;
+    const int16_t* rIe = (live_g & bei ? ringI + ((s - ei) & ri) * rowlen : none_row) + 1;
+    const int16_t* rDe = (live_g & bed ? ringD + ((s - ed) & rd) * rowlen : none_row) - 1;
+    int16_t* wM = ringM + sm * rowlen;
+    int16_t* wI = ringI + (s & ri) * rowlen;
+    int16_t* wD = ringD + (s & rd) * rowlen;
+    int* hs = TB ? hist + s * W - base : nullptr;
+    int kd = INT32_MAX, mad = INT32_MIN;  // lowest done diagonal; prune_wavefront's maximum
+    int top_m = kNone16, top_g = kNone16;
+    for (int k = alive ? lo + gl : INT32_MAX; k <= hi; k += G) {
+      int vi = kNone16, vd = kNone16, vm = 0, from = 0;
+      if (s > 0) {
+        const int i0 = rMoi[k], i1 = rIe[k], d0 = rMod[k], d1 = rDe[k], m0 = rMx[k];
+        const int io = i0 < m ? i0 + 1 : kNone16, dop = d0 <= n - k ? d0 : kNone16;
+        vi = max(io, i1 < m ? i1 + 1 : kNone16);
+        vd = max(dop, d1 <= n - k ? d1 : kNone16);
+        vm = m0 < min(m, n - k) ? m0 + 1 : kNone16;
+        top_g = max(top_g, max(vi, vd));
+        if (TB)
+          from = (vm >= max(vi, vd) ? 0 : vi >= vd ? kFromI : kFromD) | (io == vi ? kIOpen : 0) |
+                 (dop == vd ? kDOpen : 0);
+        vm = max(vm, max(vi, vd));
+      }
+      if (vm >= 0) {
+        if (TB) hs[k] = vm << 4 | from;
+        vm = kWide ? wfa_extend_wide(pw, tw, m, n, k, vm) : wfa_extend(pw, tw, m, n, k, vm);
+        mad = max(mad, 2 * vm + k);
+        if (vm >= m) kd = min(kd, k);
+      }
+      top_m = max(top_m, vm);
+      wM[k] = (int16_t)vm;
+      wI[k] = (int16_t)vi;
+      wD[k] = (int16_t)vd;
+    }
+    if (L.drop >= 0) {  // prune_wavefront (wfa.rs:293-346) on the extended M
+      __syncwarp();
+#pragma unroll
+      for (int d = 1; d < G; d <<= 1) mad = max(mad, __shfl_xor_sync(kFull, mad, d));
+      kd = INT32_MAX;
+      for (int k = alive ? lo + gl : INT32_MAX; k <= hi; k += G) {
+        const int vm = wM[k];
+        if (vm < 0) continue;
+        if (2 * vm + k < mad - L.drop) {
+          wM[k] = (int16_t)kNone16;
+        } else if (vm >= m) {
+          kd = min(kd, k);
+        }
+      }
+    }
+    __syncwarp();
+    const unsigned any_m = __ballot_sync(kFull, top_m >= 0) & gmask;
+    const unsigned any_g = __ballot_sync(kFull, top_g >= 0) & gmask;
+    if (__any_sync(kFull, kd != INT32_MAX)) {
+#pragma unroll
+      for (int d = 1; d < G; d <<= 1) kd = min(kd, __shfl_xor_sync(kFull, kd, d));
+    }
+    if (alive) {
+      live_m = live_m << 1 | (Mask)(any_m != 0), live_g = live_g << 1 | (Mask)(any_g != 0);
+      dead = (live_m & in_ring) == 0;
       if (kd != INT32_MAX) {
         done_s = s;
         k_end = kd;
-        break;
-      }
-      // Nothing reached within the look-back window: no later score reaches anything.
-      if (live) last_live = s;
-      else if (s - last_live > L.lookback) {
-        dead = true;
-        break;
-      }
-      if (++slot == R) slot = 0;
-    }
-    if (lane == 0) {
-      if (done_s < 0 && !dead && S_loop > s_lim) {
-        L.fb_list[atomicAdd(L.fb_count, 1u)] = p;  // the general kernel redoes it
+        alive = false;
+      } else if (dead || s == s_lim) {
+        alive = false;
       } else {
-        kira_wfa_result res{};
-        res.cost = -1;
-        uint32_t nops = 0;
-        if (done_s >= 0) {
-          res.found = 1;
-          res.cost = done_s;
-          res.score = L.scored ? m * L.match - done_s : done_s;
-          res.text_end = (uint32_t)(m + k_end);
-          if (TB) {
-            auto get = [&](int layer, int sc, int kk) -> int {
-              if (sc < 0 || kk < base || kk > base + kW - 1) return kWfaNone;
-              const int v = hist[(size_t)sc * 3 * kW + layer * kW + (kk - base)];
-              return v >= 0 ? v : kWfaNone;
-            };
-            bool ovf = false;
-            uint32_t* sl = L.slots + (size_t)p * L.slot_cap;
-            const int k0 = wfa_traceback_t(L, get, pw, tw, m, n, done_s, k_end, sl, nops, ovf);
-            res.text_start = (uint32_t)max(k0, 0);
-            if (ovf) atomicOr(L.flags, 1u);
-          }
-        }
-        if (TB) L.ncig[p] = nops;
-        L.out[p] = res;
+        advance();
       }
     }
-    __syncwarp();
   }
 }
 
@@ -645,24 +759,36 @@ cudaError_t launch_wfa(const DevPairs& P, const WfaLaunch& L, uint32_t blocks,
   return cudaGetLastError();
 }
 
-cudaError_t wfa_window_blocks_per_sm(int segments, bool traceback, size_t smem, int* per_sm) {
-  auto kern = segments == 4 ? (traceback ? wfa_window_kernel<4, true> : wfa_window_kernel<4, false>)
-                            : (traceback ? wfa_window_kernel<2, true> : wfa_window_kernel<2, false>);
+using WfaWindowKernel = void (*)(DevPairs, WfaLaunch, WfaWindow);
+
+template <int G>
+static WfaWindowKernel wfa_window_pick(bool traceback, bool small) {
+  return traceback ? (small ? wfa_window_kernel<G, true, uint32_t> : wfa_window_kernel<G, true, uint64_t>)
+                   : (small ? wfa_window_kernel<G, false, uint32_t> : wfa_window_kernel<G, false, uint64_t>);
+}
+
+// The row masks take 32 bits where the recurrence looks back less than 32 rows.
+static WfaWindowKernel wfa_window_pick(const WfaLaunch& L, const WfaWindow& X, bool traceback) {
+  const bool small = L.lookback < 32;
+  switch (X.lanes) {
+    case 16: return wfa_window_pick<16>(traceback, small);
+    default: return wfa_window_pick<32>(traceback, small);
+  }
+}
+
+cudaError_t wfa_window_blocks_per_sm(const WfaLaunch& L, const WfaWindow& X, bool traceback,
+                                     int* per_sm) {
+  const size_t smem = (size_t)wfa_window_pairs(X) * X.group_bytes;
+  auto kern = wfa_window_pick(L, X, traceback);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kern, 128, smem);
 }
 
-cudaError_t launch_wfa_window(const DevPairs& P, const WfaLaunch& L, uint32_t blocks,
-                              bool traceback, cudaStream_t st) {
-  const size_t smem = (size_t)4 * (L.win_ring_bytes + L.smem_group - L.ring_bytes);
-  if (L.win_segments == 4) {
-    if (traceback) (wfa_window_kernel<4, true><<<blocks, 128, smem, st>>>(P, L), count_launch());
-    else (wfa_window_kernel<4, false><<<blocks, 128, smem, st>>>(P, L), count_launch());
-  } else {
-    if (traceback) (wfa_window_kernel<2, true><<<blocks, 128, smem, st>>>(P, L), count_launch());
-    else (wfa_window_kernel<2, false><<<blocks, 128, smem, st>>>(P, L), count_launch());
-  }
+cudaError_t launch_wfa_window(const DevPairs& P, const WfaLaunch& L, const WfaWindow& X,
+                              uint32_t blocks, bool traceback, cudaStream_t st) {
+  const size_t smem = (size_t)wfa_window_pairs(X) * X.group_bytes;
+  (wfa_window_pick(L, X, traceback)<<<blocks, 128, smem, st>>>(P, L, X), count_launch());
   return cudaGetLastError();
 }
 

@@ -1,5 +1,4 @@
-// wfa.cuh -- wavefront alignment (src/alignment/wfa.rs), one (read, window) pair
-// per warp.
+// wfa.cuh -- wavefront alignment (src/alignment/wfa.rs) of (read, window) pairs.
 //
 // The recurrence is the reference's: per score s three wavefronts M, I, D hold
 // the furthest pattern offset reached on each diagonal k = j - i,
@@ -11,7 +10,8 @@
 // extend_wavefront (:277-291), prune_wavefront (:293-346), check_done (:348-358),
 // build_cigar (:762-952).
 //
-// B200 mapping: the 32 lanes of a warp own 32 consecutive diagonals of a score
+// General kernel (pairs whose fronts outgrow the window kernel's, and every pair where
+// that does not apply): the 32 lanes of a warp own 32 consecutive diagonals of a score
 // step (chunks of 32 for wider fronts), so the sources of a chunk are 64-byte
 // coalesced int16 loads and the extension of each diagonal runs in its own lane
 // over the pair's bytes staged in shared memory (8 bytes per compare). Offsets
@@ -21,7 +21,7 @@
 // trimmed to its first and last reached diagonal; the trimmed-away diagonals
 // read as "none" exactly like diagonals outside the reference's range, so no
 // offset changes. The traceback walks back in lane 0 with the reference's edge
-// order, comparing matches 4 bytes at a time.
+// order.
 #pragma once
 
 #include "common.cuh"
@@ -84,25 +84,6 @@ __device__ __forceinline__ int wfa_extend(const uint32_t* pw, const uint32_t* tw
     run += 8;
   }
   return v + max(0, min(run, lim));
-}
-
-// Backward match walk of the traceback (wfa.rs:807-853): from offset `off` on
-// diagonal k, the number of consecutive equal bytes pattern[w-1] == text[w-1+k]
-// for w = off, off-1, ..., never passing below `low`.
-__device__ __forceinline__ int wfa_back_run(const uint32_t* pw, const uint32_t* tw, int k, int off,
-                                            int low) {
-  const int lim = off - low;
-  int run = 0;
-  while (run < lim) {
-    const int p = off - run - 4;
-    const uint32_t d = wfa_ld4(pw, p) ^ wfa_ld4(tw, p + k);
-    if (d) {
-      run += __clz(d) >> 3;
-      break;
-    }
-    run += 4;
-  }
-  return max(0, min(run, lim));
 }
 
 }  // namespace kira
