@@ -1702,11 +1702,14 @@ DevPairs chunk_view(const DevPairs& D, uint32_t lo, uint32_t m) {
 }
 
 // Chunk size of a host batch: the context's setting (-1: a quarter of the batch,
-// at least 2^18 pairs; 0: one shot); chunking needs at least two chunks and no
-// stage profiling.
+// at least 2^17 pairs; 0: one shot); chunking needs at least two chunks and no
+// stage profiling. From 2^18 pairs on the overlap is worth more than the smaller
+// launches cost: prefilter of 262k / 300k / 400k pairs 1.82 / 2.11 / 2.76 ms in one
+// shot, 1.58 / 1.65 / 2.21 in chunks; WFA of 262k / 300k / 400k 3.07 / 3.37 / 4.27 and
+// 2.94 / 3.12 / 3.98; of 200k in two 2.46 and 2.57.
 uint64_t host_chunk(const kira_ctx* ctx, uint32_t n) {
   if (ctx->profile) return 0;
-  const uint64_t chunk = ctx->chunk_pairs < 0 ? std::max<uint64_t>(1u << 18, (n + 3ull) / 4)
+  const uint64_t chunk = ctx->chunk_pairs < 0 ? std::max<uint64_t>(1u << 17, (n + 3ull) / 4)
                                               : (uint64_t)ctx->chunk_pairs;
   return chunk && n >= 2 * chunk ? chunk : 0;
 }
@@ -1729,7 +1732,8 @@ int verify_host(kira_ctx* ctx, const kira_pairs& P, const kira_verify_params& pr
   // (each pays some fixed launch and tail cost). Automatic: batches of at least
   // 2^20 pairs in chunks of 1/8, 1/4, 1/4, 1/4, 1/8 of the batch (a small first
   // chunk starts the GPU sooner, a small last one drains sooner), smaller ones in
-  // quarters of at least 2^18 pairs; chunk_pairs > 0: equal chunks of that size.
+  // quarters of at least 2^17 pairs (262k / 320k / 520k pairs: 0.80 / 1.15 / 1.25 ms,
+  // in one shot 1.38 / 1.49 / 1.93); chunk_pairs > 0: equal chunks of that size.
   std::vector<uint32_t> bounds;
   if (!ctx->profile) {
     const uint64_t n = P.n;
@@ -1737,7 +1741,7 @@ int verify_host(kira_ctx* ctx, const kira_pairs& P, const kira_verify_params& pr
       bounds = {0u, (uint32_t)(n / 8), (uint32_t)(3 * n / 8), (uint32_t)(5 * n / 8),
                 (uint32_t)(n - n / 8), (uint32_t)n};
     } else {
-      const uint64_t chunk = ctx->chunk_pairs < 0 ? std::max<uint64_t>(1u << 18, (n + 3) / 4)
+      const uint64_t chunk = ctx->chunk_pairs < 0 ? std::max<uint64_t>(1u << 17, (n + 3) / 4)
                                                   : (uint64_t)ctx->chunk_pairs;
       if (chunk && n >= 2 * chunk)
         for (uint64_t lo = 0; lo <= n; lo += chunk) bounds.push_back((uint32_t)std::min(lo, n));
