@@ -1196,8 +1196,9 @@ def roofline_block(args, L, local, stage_ms, statuses, cells_step, n, tuning):
     qp, wp = (q + 3) // 4, (wl + 3) // 4
     # Algorithmic bytes per launch of each stage: 2-bit packed sequences and result
     # rows for the sieve and Myers; for the DP the ASCII read and window of every SW
-    # pair, its end coordinates, and a 4-bit trace code per executed band cell.
-    alg = {0: n * (qp + wp + 12), 1: n_my * (qp + wp + 8), 2: n_sw * (q + wl + 16) + cells_step // 2,
+    # pair, its end coordinates, and a trace byte (int32 lanes: four bits) per executed
+    # band cell.
+    alg = {0: n * (qp + wp + 12), 1: n_my * (qp + wp + 8), 2: n_sw * (q + wl + 16) + cells_step // (1 if packed else 2),
            3: n_sw * (32 + 16) + cells_step // 50, 4: n * (32 + 8) + 4 * n}
     achieved = alg[dom] / (dom_ms / 1e3) / 1e9 if dom_ms > 0 else 0.0
     per_cell = profile_figure("bsw16_dp_batched_800k.md" if packed else "bsw_dp_batched_800k.md",

@@ -306,9 +306,9 @@ typedef struct kira_verify_params {
   int32_t flags;           /* KIRA_VERIFY_* bits */
 } kira_verify_params;
 
-/* kira_verify_params.flags: turn off the exact 4-gram prefilter in front of the
+/* kira_verify_params.flags: turn off the exact block filter in front of the
  * Myers stage. The filter only removes pairs whose edit distance provably
- * exceeds k (q-gram lemma), so results are identical either way. */
+ * exceeds k, so results are identical either way. */
 #define KIRA_VERIFY_NO_QGRAM 1
 
 /* Optional per-stage detail. */

@@ -105,7 +105,7 @@ class VerifyParams:
     sieve_threshold: int = 12
     myers_k: int = 8
     cert_strict: bool = False
-    qgram_filter: bool = True  # exact 4-gram prefilter before Myers (same results)
+    qgram_filter: bool = True  # exact block filter before Myers (same results)
 
     def to_c(self) -> A.VerifyParams:
         return A.VerifyParams(self.cfg.to_c(), self.sieve_threshold, self.myers_k,
