@@ -2726,7 +2726,9 @@ int kira_gpu_ref_upload(kira_ctx* ctx, const uint8_t* seq, uint64_t len) {
   });
   ctx->ref_dev = dev;
   ctx->ref_planes = planes;
-  KIRA_CUDA(cudaMemcpy(ctx->ref_dev, seq, len, cudaMemcpyHostToDevice));
+  // On the stream that packs the planes: a plain cudaMemcpy from pageable memory may
+  // return before its last bytes have landed, and this stream does not wait for it.
+  KIRA_CUDA(cudaMemcpyAsync(ctx->ref_dev, seq, len, cudaMemcpyHostToDevice, ctx->stream));
   KIRA_CUDA(cudaMemsetAsync(ctx->ref_dev + len, 0, 16, ctx->stream));
   KIRA_CUDA(launch_pack_planes(ctx->ref_dev, len, ctx->ref_planes, nb, ctx->sms, ctx->stream));
   KIRA_CUDA(cudaStreamSynchronize(ctx->stream));
