@@ -1512,7 +1512,10 @@ template <class F>
 cudaError_t run_as_graph(kira_ctx* ctx, const DevPairs& D, const BucketRun& R,
                          const CompactLaunch& CL, const uint64_t* total_dev, cudaStream_t st,
                          F&& enqueue) {
-  // Key: every value the launches read, field by field (struct padding excluded).
+  // Key: every value the launches read, field by field (struct padding excluded), and
+  // where every device buffer of the context lies: one that another call has grown since
+  // the capture (the rescue's and the scan's are sized by more than this batch) makes a
+  // new key.
   std::vector<uint8_t> key;
   auto put = [&key](const auto& v) {
     const uint8_t* b = reinterpret_cast<const uint8_t*>(&v);
@@ -1533,6 +1536,8 @@ cudaError_t run_as_graph(kira_ctx* ctx, const DevPairs& D, const BucketRun& R,
   }
   put(CL.n), put(CL.out), put(CL.ncig), put(CL.off), put(CL.item_of_pair), put(CL.slots);
   put(CL.slot_cap), put(CL.ops), put(CL.cap), put(total_dev);
+  put(R.all.max_q), put(R.all.rescue_slots), put(R.all.rescue_slot_bytes);
+  for (const DevBuf& b : ctx->bufs) put(b.p);
   if (ctx->graph_exec && key == ctx->graph_key) {
     ++ctx->graph_replays;
     count_launch(ctx->graph_kernels);
