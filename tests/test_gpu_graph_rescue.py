@@ -40,7 +40,7 @@ def _equal(ctx, cases, cfg):
 @pytest.mark.parametrize("sizes,small,grow", [
     ((6000, 150), (60, 300), (20, 480)),      # longer reads: the rescue's trace and rows
     ((8100, 60), (8100, 60), (8200, 60))])    # one more block of the CIGAR scan
-@pytest.mark.parametrize("scoring", [(1, 4, 6, 1), (26, 200, 0, 0)])
+@pytest.mark.parametrize("scoring", [(1, 4, 6, 1), (5, 100, 0, 0)])
 def test_a_grown_buffer_recaptures(sizes, small, grow, scoring):
     from kira_ls_aligner_b200 import AlignmentConfig, GpuContext, _abi
     cfg = AlignmentConfig(*scoring, 33, 100, 5, True, 16)
