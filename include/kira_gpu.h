@@ -212,9 +212,14 @@ int kira_gpu_stage_times(kira_ctx* ctx, float* ms, int max_stages);
  * output array may be null); kira_gpu_set_bsw_shape installs a shape for every
  * band in band's class (<=16, 33, 64, 128, 256, 511; -1 restores the default
  * pick). The autotuner (Python runtime) times the shapes that cover a band on a
- * sample and installs the fastest. */
+ * sample and installs the fastest. kira_gpu_bsw_default_shape gives the shape that
+ * `items` pairs run on while none is installed (any output may be null): its index,
+ * past the listed ones for shapes that only the default pick uses, or -1 when `cfg` is
+ * outside the entry points' domain. It needs no device. */
 int kira_gpu_bsw_shapes(int* lanes, int* cells, int* packed, int max_shapes);
 int kira_gpu_set_bsw_shape(kira_ctx* ctx, uint32_t band, int shape);
+int kira_gpu_bsw_default_shape(const kira_sw_cfg* cfg, uint32_t max_band, uint32_t max_read_len,
+                               uint32_t items, int* lanes, int* cells, int* packed);
 
 /* kira_gpu_bsw_batch buckets pairs by band class (one tuned launch shape and trace
  * geometry per class, longest reads first, dynamic work fetching). plain = 1

@@ -36,7 +36,8 @@ EXPORTS = (
     "kira_gpu_arena_bytes", "kira_gpu_sieve_batch", "kira_gpu_ref_upload",
     "kira_gpu_myers_batch", "kira_gpu_bsw_batch", "kira_gpu_verify_batch",
     "kira_gpu_verify_dev", "kira_gpu_profile", "kira_gpu_stage_times",
-    "kira_gpu_bsw_shapes", "kira_gpu_set_bsw_shape", "kira_gpu_bsw_batch_noalloc",
+    "kira_gpu_bsw_shapes", "kira_gpu_set_bsw_shape", "kira_gpu_bsw_default_shape",
+    "kira_gpu_bsw_batch_noalloc",
     "kira_gpu_align_batch_simd", "kira_gpu_set_plain", "kira_gpu_set_trace_budget",
     "kira_gpu_set_graphs", "kira_gpu_set_chunk_pairs", "kira_gpu_nm_md", "kira_gpu_wfa_batch",
     "kira_gpu_set_wfa_lanes", "kira_gpu_prefilter_batch", "kira_gpu_exact_match_batch",
@@ -178,6 +179,7 @@ def lib():
                                       C.c_uint64, vp, vp, vp, vp]
     L.kira_gpu_profile.argtypes = [vp, C.c_int]
     L.kira_gpu_bsw_shapes.argtypes = [vp, vp, vp, C.c_int]
+    L.kira_gpu_bsw_default_shape.argtypes = [vp, C.c_uint32, C.c_uint32, C.c_uint32, vp, vp, vp]
     L.kira_gpu_set_plain.argtypes = [vp, C.c_int]
     L.kira_gpu_set_trace_budget.argtypes = [vp, C.c_uint64]
     L.kira_gpu_set_graphs.argtypes = [vp, C.c_int, vp, vp]

@@ -278,7 +278,7 @@ int plain_shape(uint32_t max_band) {
 }
 
 bool shape_fits(int s, uint32_t max_band) {
-  return s >= 0 && s < kNumAllBswShapes &&
+  return s >= 0 && s < kNumBandedBswShapes &&
          shape_cap(kBswShapes[s]) >= 2 * (int)std::max<uint32_t>(max_band, 1) + 1;
 }
 
@@ -295,24 +295,34 @@ bool shape_usable(int s, uint32_t max_band, uint32_t max_q, const SwParams& sp) 
 // exchange), more lanes finish a row sooner. Measured DP times at 150 bp, band 33 (1 x 34
 // words, 4 x 9, 8 x 5, 32 x 2): 100,000 items 0.79 / 1.18 / 1.73 / 4.34 ms; 20,000 items
 // 0.29 / 0.29 / 0.37 / 0.90; 8,000 items 0.23 / 0.17 / 0.18 / 0.37; 2,000 items 0.21 /
-// 0.15 / 0.10 / 0.12; 16 items 0.17 / 0.14 / 0.10 / 0.06. Batches no pick fits take any
-// packed shape that does, else the int32 shape of the one-launch path.
+// 0.15 / 0.10 / 0.12; 16 items 0.17 / 0.14 / 0.10 / 0.06. The other lines, DP and traceback
+// in us on both sides (at 300 bp, and 1,000 where it fits, they cross at the same counts):
+//   band 17, 2 x 9 / 4 x 5 words: 12,000 items 192 / 172, 16,000 203 / 206, 24,000 247 / 312,
+//     100,000 796 / 1037; 1 x 34 / 4 x 5 (bands 18 and 19): 30,000 391 / 362, 100,000 987 / 1037
+//   band 50, 32 x 2 / 8 x 9: 1,700 items 101 / 120, 2,200 122 / 119, 3,400 162 / 146, 100,000
+//     3905 / 2085
+//   band 50 and 64, 8 x 9 / 2 x 34: 30,000 items 660 / 780, 40,000 891 / 931, 50,000 1075 /
+//     1055, 100,000 2085 / 1926
+//   band 64, 8 x 9 / 16 x 9: 1,200 items 118 / 133
+//   band 100, 16 x 9 / 4 x 34: 6,000 items 311 / 326, 7,500 380 / 338, 9,000 412 / 344
+// Batches no pick fits take any packed shape that does, else the int32 shape of the
+// one-launch path.
 int default_shape(uint32_t max_band, uint32_t max_q, const SwParams& sp, uint32_t items) {
   struct Pick {
     int shape;
     uint32_t min_items;
   };
   constexpr Pick kPicks[] = {
-      {23, 20000}, {8, 8000},                // 34 cells on 1 lane, 40 on 4
-      {22, 20000}, {9, 8000},   {10, 1200},  // 68 on 1, 72 on 4, 80 on 8
-      {24, 0},                               // 128 on 32
-      {19, 20000}, {11, 1200},               // 136 on 2, 144 on 8
-      {20, 10000}, {12, 1200},               // 272 on 4, 288 on 16
-      {25, 0},     {13, 0},                  // 320 and 576 on 32
+      {23, 20000}, {7, 18000},                        // 34 cells on 1 lane, 36 on 2
+      {22, 60000}, {8, 8000},                         // 68 on 1, 40 on 4
+      {22, 20000}, {9, 8000},  {10, 1200},            // 68 on 1, 72 on 4, 80 on 8
+      {19, 50000}, {11, 2000}, {24, 0},   {11, 1200},  // 136 on 2, 144 on 8, 128 on 32
+      {20, 7000},  {12, 1200},                        // 272 on 4, 288 on 16
+      {25, 0},     {13, 0},                           // 320 and 576 on 32
   };
   for (const Pick& p : kPicks)
     if (items >= p.min_items && shape_usable(p.shape, max_band, max_q, sp)) return p.shape;
-  for (int s = 0; s < kNumAllBswShapes; ++s)
+  for (int s = 0; s < kNumBandedBswShapes; ++s)
     if (kBswShapes[s].packed && shape_usable(s, max_band, max_q, sp)) return s;
   return plain_shape(max_band);
 }
@@ -2681,6 +2691,17 @@ int kira_gpu_bsw_shapes(int* lanes, int* cells, int* packed, int max_shapes) {
     if (packed) packed[i] = kBswShapes[i].packed;
   }
   return kNumBswShapes;
+}
+
+int kira_gpu_bsw_default_shape(const kira_sw_cfg* cfg, uint32_t max_band, uint32_t max_read_len,
+                               uint32_t items, int* lanes, int* cells, int* packed) {
+  if (!cfg || sw_cfg_problem(*cfg, max_read_len, max_band)) return -1;
+  const int s = default_shape(max_band, max_read_len, resolve(*cfg), items);
+  if (s < 0) return -1;
+  if (lanes) *lanes = kBswShapes[s].g;
+  if (cells) *cells = shape_cap(kBswShapes[s]) / kBswShapes[s].g;
+  if (packed) *packed = kBswShapes[s].packed;
+  return s;
 }
 
 int kira_gpu_profile(kira_ctx* ctx, int enable) {

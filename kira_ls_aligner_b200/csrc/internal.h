@@ -234,7 +234,8 @@ struct BswShapeInfo {
 };
 extern const BswShapeInfo kBswShapes[];
 extern const int kNumBswShapes;     // the listed shapes (kira_gpu_bsw_shapes)
-extern const int kNumAllBswShapes;  // and the ones only the default pick uses, after them
+extern const int kNumBandedBswShapes;  // and the ones only the default pick uses, after them
+                                       // (past those: full-window sweeps alone)
 
 inline int shape_cap(const BswShapeInfo& s) { return (s.packed ? 2 : 1) * s.g * s.k; }
 inline uint32_t shape_lane_bytes(const BswShapeInfo& s) {

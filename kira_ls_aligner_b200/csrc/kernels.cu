@@ -1091,11 +1091,12 @@ const BswShapeInfo kBswShapes[] = {
     // a warp per pair with the fewest words a lane, for the shortest rows: bands up to
     // 63 and 159
     {32, 2, 32, 16, 1},  {32, 5, 32, 16, 1},
-    // full-window batches: windows up to 272 and 544 on 17 words a lane
+    // ---- no banded sweep (kNumBandedBswShapes): full-window batches, windows up to 272
+    // and 544 on 17 words a lane
     {8, 17, 32, 16, 1},  {16, 17, 32, 16, 1},
 };
 const int kNumBswShapes = 23;
-const int kNumAllBswShapes = sizeof(kBswShapes) / sizeof(kBswShapes[0]);
+const int kNumBandedBswShapes = 26;
 
 cudaError_t launch_bsw(int shape, const DevPairs& P, const BswLaunch& B, uint32_t max_items,
                        int sms, cudaStream_t st, cudaEvent_t between, int parts) {
