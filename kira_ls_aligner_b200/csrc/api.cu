@@ -239,6 +239,16 @@ SwParams resolve(const kira_sw_cfg& c) {
   return s;
 }
 
+// The banded SW's parameters on reads of up to max_q bases. A mismatch above the highest
+// score ends every alignment, whatever its size: it is cut to one more than that score,
+// which keeps the values of scorings that forbid mismatches small.
+SwParams resolve(const kira_sw_cfg& c, uint32_t max_q) {
+  SwParams s = resolve(c);
+  s.mismatch = (int32_t)std::min<int64_t>(s.mismatch,
+                                          (int64_t)max_q * std::max(s.match, 0) + 1);
+  return s;
+}
+
 // Domain of the GPU banded SW (exactness conditions of the F prefix scan and of
 // the packed row-argmax key).
 }  // namespace
@@ -639,7 +649,7 @@ int verify_pipeline(kira_ctx* ctx, DevPairs D, const Maxes& mx, const kira_verif
   int rc = check_sw_cfg(ctx, p.sw, mx.q, mx.band);
   if (rc) return rc;
   if (mx.q > 512) return fail(ctx, KIRA_ERR_READ_TOO_LONG, "read of %u bases > 512", mx.q);
-  const SwParams sp = resolve(p.sw);
+  const SwParams sp = resolve(p.sw, mx.q);
   const int shape = pick_shape(ctx, mx.band, mx.q, sp, expected_sw_items(n));
   if (shape < 0) return fail(ctx, KIRA_ERR_INVALID, "no banded-SW shape for band %u", mx.band);
   uint32_t* ncig = df ? df->ncig + df->base : nullptr;
@@ -656,7 +666,7 @@ int verify_pipeline(kira_ctx* ctx, DevPairs D, const Maxes& mx, const kira_verif
   KIRA_DBUF(mlist, uint32_t, B_MYERS_LIST, n);
   KIRA_DBUF(counters, uint32_t, B_COUNTERS, 4);
   KIRA_CUDA(cudaMemsetAsync(counters, 0, cm.first ? 16 : 8, st));
-  VerifyDev V{p.sieve_threshold, p.cert_strict, sp,       out,       detail, ncig,
+  VerifyDev V{p.sieve_threshold, p.cert_strict, resolve(p.sw), out,       detail, ncig,
               swoff,             mlist,         counters, p.myers_k, (p.flags & KIRA_VERIFY_NO_QGRAM) ? 0 : 1,
               nullptr,           nullptr,       slist,    df ? df->count : counters + 1,
               df ? df->base : 0u};
@@ -882,7 +892,7 @@ int plan_bucketed(kira_ctx* ctx, const kira_pairs& P, const DevPairs& D, const k
       std::stable_sort(list.begin() + base[c], list.begin() + base[c + 1],
                        [&](uint32_t a, uint32_t b) { return P.read_len[a] > P.read_len[b]; });
   }
-  const SwParams sp = resolve(cfg);
+  const SwParams sp = resolve(cfg, qall);
   int shape[kBandClasses];
   uint64_t slot[kBandClasses] = {}, per[kBandClasses] = {};
   uint64_t total = 0;
@@ -1305,7 +1315,6 @@ int verify_batch_chunked(kira_ctx* ctx, const kira_pairs& P, const kira_verify_p
     if (!ctx->ev_cls_fork)
       KIRA_CUDA(cudaEventCreateWithFlags(&ctx->ev_cls_fork, cudaEventDisableTiming));
   }
-  const SwParams gsp = resolve(p.sw);
   BswLaunch gB[2] = {};
   // DP + traceback of group g (chunks [c0, c1)) on side streams 2g and 2g + 1,
   // behind the group's front stages; ev_cls_join[g] marks the end.
@@ -1318,6 +1327,7 @@ int verify_batch_chunked(kira_ctx* ctx, const kira_pairs& P, const kira_verify_p
       gm.w = std::max(gm.w, scans[c].mx.w);
       gm.band = std::max(gm.band, scans[c].mx.band);
     }
+    const SwParams gsp = resolve(p.sw, gm.q);
     const uint32_t lo = bounds[c0], ng = bounds[c1] - lo;
     const int shape = pick_shape(ctx, gm.band, gm.q, gsp, expected_sw_items(ng));
     if (shape < 0) return fail(ctx, KIRA_ERR_INVALID, "no banded-SW shape for band %u", gm.band);
@@ -2696,7 +2706,7 @@ int kira_gpu_bsw_shapes(int* lanes, int* cells, int* packed, int max_shapes) {
 int kira_gpu_bsw_default_shape(const kira_sw_cfg* cfg, uint32_t max_band, uint32_t max_read_len,
                                uint32_t items, int* lanes, int* cells, int* packed) {
   if (!cfg || sw_cfg_problem(*cfg, max_read_len, max_band)) return -1;
-  const int s = default_shape(max_band, max_read_len, resolve(*cfg), items);
+  const int s = default_shape(max_band, max_read_len, resolve(*cfg, max_read_len), items);
   if (s < 0) return -1;
   if (lanes) *lanes = kBswShapes[s].g;
   if (cells) *cells = shape_cap(kBswShapes[s]) / kBswShapes[s].g;
@@ -2831,7 +2841,7 @@ int kira_gpu_bsw_batch(kira_ctx* ctx, const kira_pairs* pairs, const kira_sw_cfg
     // the batch's widest band (the tuned shape of its class when the batch fits it,
     // packed int16 wherever the scores fit, else int32), one launch over every pair
     // in input order; only the bucketing, dynamic fetch and graph replay differ.
-    const SwParams sp = resolve(*cfg);
+    const SwParams sp = resolve(*cfg, mx.q);
     const int shape = pick_shape(ctx, mx.band, mx.q, sp, n);
     if (shape < 0)
       return fail(ctx, KIRA_ERR_INVALID, "band %u above the one-launch maximum", mx.band);
@@ -2944,7 +2954,7 @@ int kira_gpu_align_batch_simd(kira_ctx* ctx, const kira_pairs* pairs, const kira
   // itself (no rescue in this mode), else int32. Eight lanes a pair and more words each do
   // less work, a warp per pair finishes a row sooner.
   const int cap_need = (int)r0;
-  const SwParams fsp = resolve(*cfg);
+  const SwParams fsp = resolve(*cfg, q0);
   int shape = -1;
   if (!packed_trace_wraps(q0, fsp)) {
     constexpr int kMany[] = {10, 11, 26, 27}, kFew[] = {24, 25, 13};

@@ -275,11 +275,32 @@ inline int packed_key_bits(int k) {
   return k <= 2 ? 1 : k <= 4 ? 2 : k <= 8 ? 3 : k <= 16 ? 4 : k <= 32 ? 5 : 6;
 }
 
+// The packed trace keeps H mod 256. A walk's comparisons are between values of at most
+// max_q * match and differ from them by a mismatch or one gap step: it can lose its
+// value only when those pass 255.
+inline bool packed_trace_wraps(uint32_t max_q, const SwParams& sp) {
+  return (int64_t)max_q * sp.match + std::max(sp.mismatch, sp.gof + sp.gap_extend) > 255;
+}
+
+// Scorings on which a wrapped trace goes wrong in the middle of a band. Where the cells
+// around it are in band, the diagonal predecessor's H lies in [v - match, v + 2 gof] of a
+// cell of value v (two gap steps join them, and an alignment cut by its last column and row
+// loses at most a match), so the diagonal is taken wrongly when mismatch is a multiple of
+// 256 plus something of [-match, 2 gof]: 100,000 pairs of 150 bp at match 9, mismatch 247,
+// gaps 0 and 3 lost nearly all their walks and took 4.4 s, on int32 lanes 4.9 ms. What
+// remains is left to the rescue: a jump at the band's edge, or a gap cell 256 below what the gap needs (1 in 100 to
+// 1 in 6,000 short noisy reads on scorings of 10 to 30 a match, none on the default's).
+inline bool packed_trace_aliases(const SwParams& sp) {
+  const int64_t step = (int64_t)sp.match + sp.mismatch;
+  return step > 255 && step % 256 <= sp.match + 2ll * sp.gof;
+}
+
 // The packed sweep is exact when every biased value stays below 2^13 and every biased H
-// fits a row-max key (H << key bits below 2^16).
+// fits a row-max key (H << key bits below 2^16); its trace has to be readable too.
 inline bool packed_fits(const BswShapeInfo& s, uint32_t max_q, const SwParams& sp) {
   if (!s.packed) return false;
   if (sp.match < 0 || sp.mismatch < 0 || sp.gap_open < 0 || sp.gap_extend < 0) return false;
+  if (packed_trace_wraps(max_q, sp) && packed_trace_aliases(sp)) return false;
   const int64_t top = (int64_t)max_q * sp.match;
   const int64_t cap = shape_cap(s);
   if (top + (int64_t)packed_bias(s, sp) >= (int64_t(1) << (16 - packed_key_bits(s.k))))
@@ -321,12 +342,6 @@ cudaError_t launch_bsw_rescue(const DevPairs& P, const BswLaunch& B, cudaStream_
 // Trace row of the rescue's int32 sweep (576 cells, the widest listed row).
 constexpr int kRescueLanes = 32, kRescueCells = 18;
 constexpr uint64_t kRescueRowBytes = 4ull * kRescueLanes * ((kRescueCells + 7) / 8);
-// The packed trace keeps H mod 256. A walk's comparisons are between values of at most
-// max_q * match and differ from them by a mismatch or one gap step: it can lose its
-// value only when those pass 255.
-inline bool packed_trace_wraps(uint32_t max_q, const SwParams& sp) {
-  return (int64_t)max_q * sp.match + std::max(sp.mismatch, sp.gof + sp.gap_extend) > 255;
-}
 cudaError_t launch_cigar_scan(const uint32_t* ncig, uint32_t n, uint32_t* off,
                               uint32_t* chunk_sums, uint64_t* total_dev, cudaStream_t st,
                               bool accumulate = false);
