@@ -552,14 +552,18 @@ int prepare_bsw(kira_ctx* ctx, uint32_t n_pairs, uint32_t items, uint32_t trace_
 
 // Rescue list and trace slots of a banded-SW stage whose packed traces can wrap (`any`:
 // it has a packed shape); `count` is the list's count word, reset with the stage's
-// counters.
-constexpr uint32_t kRescueSlots = 8;
+// counters. A slot is one warp's: eight of them held up batches where one walk in a few
+// hundred is lost (200,000 noisy reads of 150 bp at band 6, match 20, mismatch 40, gaps 3 and
+// 1: 14.0 ms a call, 7.6 with these, 9.5 with the whole batch on int32 lanes).
+constexpr uint64_t kRescueBytes = 32ull << 20;
 int prepare_rescue(kira_ctx* ctx, uint32_t items, uint32_t max_q, bool any, const SwParams& sp,
                    uint32_t* count, BswLaunch& B) {
   if (!any || !packed_trace_wraps(max_q, sp)) return KIRA_OK;
   cudaError_t cerr = cudaSuccess;
-  B.rescue_slots = std::min(kRescueSlots, std::max<uint32_t>(items, 1));
   B.rescue_slot_bytes = (max_q + 1ull) * kRescueRowBytes;
+  const uint64_t slots = std::min<uint64_t>(kRescueBytes / B.rescue_slot_bytes, 4ull * ctx->sms);
+  B.rescue_slots = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(slots, 8),
+                                                std::max<uint32_t>(items, 1));
   KIRA_DBUF(list, uint32_t, B_RESCUE_LIST, std::max<uint32_t>(items, 1));
   KIRA_DBUF(trace, uint8_t, B_RESCUE_TRACE, B.rescue_slot_bytes * B.rescue_slots);
   KIRA_DBUF(meta, uint32_t, B_RESCUE_META, (max_q + 1ull) * B.rescue_slots);

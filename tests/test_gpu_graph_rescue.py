@@ -38,7 +38,7 @@ def _equal(ctx, cases, cfg):
 
 # (first batch: pairs and read length; the captured one; the call that grows)
 @pytest.mark.parametrize("sizes,small,grow", [
-    ((6000, 150), (60, 300), (20, 480)),      # longer reads: the rescue's trace and rows
+    ((6000, 150), (60, 300), (60, 480)),      # longer reads: the rescue's trace and rows
     ((8100, 60), (8100, 60), (8200, 60))])    # one more block of the CIGAR scan
 @pytest.mark.parametrize("scoring", [(1, 4, 6, 1), (5, 100, 0, 0)])
 def test_a_grown_buffer_recaptures(sizes, small, grow, scoring):
