@@ -2204,11 +2204,17 @@ int kira_gpu_wfa_batch(kira_ctx* ctx, const kira_pairs* pairs, const kira_wfa_pa
   L.slot_cap = (uint32_t)(2 * (S / min_cost) + 2);
   L.max_score_pp = nullptr;
   L.tbf_pp = nullptr;
-  // Fixed-window passes: 64 diagonals per pair, then 128 for what 64 leave open (128
-  // at once when 64 cover fewer than 32 scores), placed so every cell of the highest
-  // score stays inside for this batch's leading free text; pairs still open after
-  // that fall back to the general kernel with a warp per pair (their fronts are the
-  // wide ones). ctx->wfa_lanes != 0 forces the general kernel alone.
+  // Fixed-window passes: 64 diagonals per pair, then 128 for what 64 leave open, placed so
+  // every cell of the highest score stays inside for this batch's leading free text; pairs
+  // still open after that fall back to the general kernel with a warp per pair (their
+  // fronts are the wide ones). A pass that leaves most pairs open is work for nothing, so
+  // one whose scores end before 32, or before mismatches on a 32nd of the longest read, is
+  // left out: the 64 from about 300 bases on with the usual costs, and without a traceback
+  // the 128 too from about 600 on (20,000 reads of 400 bases, 1 / 4 % of errors at most:
+  // 0.49 / 1.67 ms with both, 0.44 / 1.49 with 128 alone; 6,000 of 1,000, no traceback: 0.90
+  // / 3.11 with both, 0.64 / 2.64 with the general kernel alone; free leading text makes
+  // that one's fronts wide from the start: 20,000 of 400 with 40 free, 1.8 against 3.3).
+  // ctx->wfa_lanes != 0 forces the general kernel alone.
   auto place = [&](int width, int* base) {
     int best = -1;
     for (int b = -(width - 1 - (int)tbf_max); b <= 0; ++b) {
@@ -2244,7 +2250,9 @@ int kira_gpu_wfa_batch(kira_ctx* ctx, const kira_pairs* pairs, const kira_wfa_pa
     int b64 = 0, b128 = 0;
     const int s64 = tbf_max <= 63 ? place(64, &b64) : -1;
     const int s128 = tbf_max <= 127 ? place(128, &b128) : -1;
-    if (s64 >= 16 && s64 >= std::min<int64_t>(S, 32)) {
+    const int64_t share = (int64_t)L.x * m_max / 32;
+    const auto serves = [&](int s) { return tb || tbf_max >= 16 || s >= std::min(S, share); };
+    if (s64 >= 16 && s64 >= std::min<int64_t>(S, std::max<int64_t>(share, 32))) {
       // 16 lanes per pair, two pairs a warp, hide each other's idle lanes (200k pairs of
       // 100 / 150 / 250 / 400 bases: 0.70 / 1.45 / 3.36 / 8.8 ms against 0.94 / 1.78 /
       // 3.83 / 9.4 with 32; with 32 free leading bases 2.15 both) while four blocks of
@@ -2252,10 +2260,10 @@ int kira_gpu_wfa_batch(kira_ctx* ctx, const kira_pairs* pairs, const kira_wfa_pa
       if (add_window(64, b64, s64, 16) > (56u << 10)) add_window(64, b64, s64, 32);
       ++wins;
     }
-    if (s128 >= 16 && (wins ? S > win[0].smax && s128 > s64 : s128 > s64)) {
+    if (s128 >= 16 && serves(s128) && (wins ? S > win[0].smax && s128 > s64 : s128 > s64)) {
       add_window(128, b128, s128, 32);
       ++wins;
-    } else if (!wins && s64 >= 16) {
+    } else if (!wins && s64 >= 16 && serves(s64)) {
       add_window(64, b64, s64, 32);
       ++wins;
     }
