@@ -2985,6 +2985,14 @@ int kira_gpu_align_batch_simd(kira_ctx* ctx, const kira_pairs* pairs, const kira
   for (int s = 0; s < kNumBswShapes && wide < 0; ++s)
     if (!kBswShapes[s].packed && shape_cap(kBswShapes[s]) >= cap_need) wide = s;
   if (shape < 0 || wide < 0) shape = wide;
+  // Every pair's trace is held at once. Past the arena's budget the int32 sweep runs, whose
+  // trace is half a byte a cell, so that a batch that fits with it is not refused.
+  if (shape >= 0 && kBswShapes[shape].packed) {
+    const uint64_t slots = trace_slot_bytes(shape, q0) * n, rows = (q0 + 1ull) * n;
+    if (trace_slot_bytes(wide, q0) * n < slots && !trace_arena_holds(ctx, slots, rows) &&
+        slots + 4 * rows > trace_budget(ctx))
+      shape = wide;
+  }
   if (shape < 0)
     return fail(ctx, KIRA_ERR_INVALID, "full-window batch: window of %u > supported 544", r0);
   if (cfg->gap_open < 0 || cfg->gap_extend < 0)
