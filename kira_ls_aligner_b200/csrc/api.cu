@@ -1382,12 +1382,18 @@ int verify_batch_chunked(kira_ctx* ctx, const kira_pairs& P, const kira_verify_p
   std::vector<uint64_t> r_from(nch), r_to(nch), w_from(nch), w_to(nch);
   uint64_t rdone = 0, wdone = 0;
   cudaStream_t up = ctx->h2d;
+  // Before an error return: what the earlier chunks (and group 0's SW on its side streams)
+  // have enqueued uses this context's buffers, which the next call may move.
+  auto drain = [&]() {
+    cudaStreamSynchronize(up);
+    cudaStreamSynchronize(st);
+    cudaStreamSynchronize(twin->stream);
+    for (int k = 0; k < 4; ++k)
+      if (ctx->cls_st[k]) cudaStreamSynchronize(ctx->cls_st[k]);
+  };
   for (uint32_t c = 0; c < nch; ++c) {
     if (int rc = checked(c)) {
-      // Earlier chunks' uploads and kernels are enqueued; let them finish first.
-      cudaStreamSynchronize(up);
-      cudaStreamSynchronize(st);
-      cudaStreamSynchronize(twin->stream);
+      drain();
       return rc;
     }
     const uint32_t lo = bounds[c], hi = bounds[c + 1], m = hi - lo;
@@ -1464,11 +1470,7 @@ int verify_batch_chunked(kira_ctx* ctx, const kira_pairs& P, const kira_verify_p
     if (!rc && grouped && c + 1 == nch) rc = run_group_sw(1, gsplit, nch);
     if (rc) {
       if (cx != ctx && cx->last_error.size()) ctx->last_error = cx->last_error;
-      cudaStreamSynchronize(up);
-      cudaStreamSynchronize(st);
-      cudaStreamSynchronize(twin->stream);
-      for (int k = 0; k < 4; ++k)
-        if (ctx->cls_st[k]) cudaStreamSynchronize(ctx->cls_st[k]);
+      drain();
       return rc;
     }
   }
