@@ -495,6 +495,11 @@ int pick_shape(const kira_ctx* ctx, uint32_t max_band, uint32_t max_q, const SwP
 // bounds.
 inline uint32_t expected_sw_items(uint32_t n) { return n / 8; }
 
+// Trace slots of that stage: a slot a pair, from 2^20 pairs on for every other pair; the
+// items past them go in a second round. (2M pairs of 150 bases: 10.4 GB of slots for 20.7,
+// the first call of a process 163 -> 108 ms; an empty second round costs about 8 us.)
+inline uint32_t sw_stage_slots(uint32_t n) { return n >= (1u << 20) ? n / 2 : n; }
+
 // Bytes the banded-SW trace arena (trace slots + row metadata) may take: the
 // context's override, else half of the free device memory plus what the arena
 // already holds, between 64 MiB and 64 GiB.
@@ -589,6 +594,31 @@ cudaError_t launch_bsw_rounds(int shape, const DevPairs& D, BswLaunch B, uint32_
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
+}
+
+// The same with the two halves of the first round on two streams at once (split on the
+// device by the item count), so that one half's DP fills the SMs the other's last wave leaves
+// idle and its traceback overlaps that DP. `s1` holds the stage before and after. Items past
+// the first round are few or none.
+cudaError_t launch_bsw_split(int shape, const DevPairs& D, BswLaunch B, uint32_t items,
+                             uint32_t per_round, int sms, cudaStream_t s1, cudaStream_t s2,
+                             cudaEvent_t fork, cudaEvent_t join) {
+  cudaError_t e = cudaEventRecord(fork, s1);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(s2, fork, 0);
+  B.item_hi = items > per_round ? per_round : 0u;
+  for (uint32_t half = 1; half <= 2 && e == cudaSuccess; ++half) {
+    B.split = half;
+    e = launch_bsw(shape, D, B, per_round, sms, half == 1 ? s1 : s2);
+  }
+  if (e == cudaSuccess) e = cudaEventRecord(join, s2);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(s1, join, 0);
+  B.split = 0;
+  for (uint32_t lo = per_round; lo < items && e == cudaSuccess; lo += per_round) {
+    B.item_lo = lo;
+    B.item_hi = lo + per_round;
+    e = launch_bsw(shape, D, B, per_round, sms, s1);
+  }
+  return e;
 }
 
 // After every traceback of a stage: the items whose packed walk was lost, if any can be.
@@ -708,7 +738,8 @@ int verify_pipeline(kira_ctx* ctx, DevPairs D, const Maxes& mx, const kira_verif
   KIRA_CUDA(launch_myers(D, M, n, ctx->sms, st));
   if (df) return KIRA_OK;  // the SW stage runs over the group's items later
   BswLaunch B{};
-  const uint32_t per_round = round_items(ctx, n, shape, mx.q);
+  const uint32_t slots = sw_stage_slots(n);
+  const uint32_t per_round = round_items(ctx, slots, shape, mx.q);
   rc = prepare_bsw(ctx, n, n, per_round, mx, shape, B);
   mark(ctx, 2, st);
   if (rc) return rc;
@@ -723,22 +754,12 @@ int verify_pipeline(kira_ctx* ctx, DevPairs D, const Maxes& mx, const kira_verif
   B.flags = counters + 2;
   rc = prepare_rescue(ctx, n, mx.q, kBswShapes[shape].packed, sp, counters + 3, B);
   if (rc) return rc;
-  if (per_round >= n && n >= kSplitPairs && !ctx->profile) {
-    // One trace round: the two halves of the banded-SW items (split on the device
-    // by the Myers stage's count) run on two streams, so one half's DP fills the
-    // SMs the other's last wave leaves idle and its traceback overlaps that DP.
+  if (per_round >= slots && n >= kSplitPairs && !ctx->profile) {
     if (!ctx->aux) KIRA_CUDA(cudaStreamCreateWithFlags(&ctx->aux, cudaStreamNonBlocking));
     if (!ctx->ev_fork) KIRA_CUDA(cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming));
     if (!ctx->ev_join) KIRA_CUDA(cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming));
-    KIRA_CUDA(cudaEventRecord(ctx->ev_fork, st));
-    KIRA_CUDA(cudaStreamWaitEvent(ctx->aux, ctx->ev_fork, 0));
-    BswLaunch B1 = B, B2 = B;
-    B1.split = 1u;
-    B2.split = 2u;
-    KIRA_CUDA(launch_bsw(shape, D, B1, n, ctx->sms, st));
-    KIRA_CUDA(launch_bsw(shape, D, B2, n, ctx->sms, ctx->aux));
-    KIRA_CUDA(cudaEventRecord(ctx->ev_join, ctx->aux));
-    KIRA_CUDA(cudaStreamWaitEvent(st, ctx->ev_join, 0));
+    KIRA_CUDA(launch_bsw_split(shape, D, B, n, per_round, ctx->sms, st, ctx->aux, ctx->ev_fork,
+                               ctx->ev_join));
   } else {
     KIRA_CUDA(launch_bsw_rounds(shape, D, B, n, per_round, ctx->sms, st,
                                 ctx->profile ? ctx->ev[3] : nullptr));
@@ -1335,7 +1356,8 @@ int verify_batch_chunked(kira_ctx* ctx, const kira_pairs& P, const kira_verify_p
     const uint32_t lo = bounds[c0], ng = bounds[c1] - lo;
     const int shape = pick_shape(ctx, gm.band, gm.q, gsp, expected_sw_items(ng));
     if (shape < 0) return fail(ctx, KIRA_ERR_INVALID, "no banded-SW shape for band %u", gm.band);
-    const uint32_t per_round = round_items(gx, ng, shape, gm.q);
+    const uint32_t slots = sw_stage_slots(ng);
+    const uint32_t per_round = round_items(gx, slots, shape, gm.q);
     BswLaunch& B = gB[g];
     int rc = prepare_bsw(gx, n, ng, per_round, gm, shape, B);
     if (rc) {
@@ -1362,16 +1384,9 @@ int verify_batch_chunked(kira_ctx* ctx, const kira_pairs& P, const kira_verify_p
     KIRA_CUDA(cudaStreamWaitEvent(s1, ctx->ev_cls_join[2 + g], 0));
     for (uint32_t c = c0; c < c1; ++c) KIRA_CUDA(cudaStreamWaitEvent(s1, ctx->ev_comp[c], 0));
     const DevPairs Dg{n,  rs, ro, rl, ws, wo, wl, bo, ab, bw, rp, wp};
-    if (per_round >= ng && ng >= kSplitPairs) {
-      KIRA_CUDA(cudaEventRecord(ctx->ev_cls_join[4 + g], s1));
-      KIRA_CUDA(cudaStreamWaitEvent(s2, ctx->ev_cls_join[4 + g], 0));
-      BswLaunch B1 = B, B2 = B;
-      B1.split = 1u;
-      B2.split = 2u;
-      KIRA_CUDA(launch_bsw(shape, Dg, B1, ng, ctx->sms, s1));
-      KIRA_CUDA(launch_bsw(shape, Dg, B2, ng, ctx->sms, s2));
-      KIRA_CUDA(cudaEventRecord(ctx->ev_cls_join[4 + g], s2));
-      KIRA_CUDA(cudaStreamWaitEvent(s1, ctx->ev_cls_join[4 + g], 0));
+    if (per_round >= slots && ng >= kSplitPairs) {
+      KIRA_CUDA(launch_bsw_split(shape, Dg, B, ng, per_round, ctx->sms, s1, s2,
+                                 ctx->ev_cls_join[4 + g], ctx->ev_cls_fork));
     } else {
       KIRA_CUDA(launch_bsw_rounds(shape, Dg, B, ng, per_round, ctx->sms, s1, nullptr));
     }
