@@ -2231,6 +2231,10 @@ int kira_gpu_wfa_batch(kira_ctx* ctx, const kira_pairs* pairs, const kira_wfa_pa
   // 0.49 / 1.67 ms with both, 0.44 / 1.49 with 128 alone; 6,000 of 1,000, no traceback: 0.90
   // / 3.11 with both, 0.64 / 2.64 with the general kernel alone; free leading text makes
   // that one's fronts wide from the start: 20,000 of 400 with 40 free, 1.8 against 3.3).
+  // A batch that does not fill the GPU waits for each pass in turn: below 2^15 pairs the 64
+  // go first only where their scores reach mismatches on a 12th of the longest read (24,000
+  // reads of 180-200 bases at 4 %: 1.55 ms with both, 1.48 with 128 alone; 1,000 of them
+  // 1.15 and 1.10).
   // ctx->wfa_lanes != 0 forces the general kernel alone.
   auto place = [&](int width, int* base) {
     int best = -1;
@@ -2269,7 +2273,8 @@ int kira_gpu_wfa_batch(kira_ctx* ctx, const kira_pairs* pairs, const kira_wfa_pa
     const int s128 = tbf_max <= 127 ? place(128, &b128) : -1;
     const int64_t share = (int64_t)L.x * m_max / 32;
     const auto serves = [&](int s) { return tb || tbf_max >= 16 || s >= std::min(S, share); };
-    if (s64 >= 16 && s64 >= std::min<int64_t>(S, std::max<int64_t>(share, 32))) {
+    const int64_t first = n < (1u << 15) ? (int64_t)L.x * m_max / 12 : share;
+    if (s64 >= 16 && s64 >= std::min<int64_t>(S, std::max<int64_t>(first, 32))) {
       // 16 lanes per pair, two pairs a warp, hide each other's idle lanes (200k pairs of
       // 100 / 150 / 250 / 400 bases: 0.70 / 1.45 / 3.36 / 8.8 ms against 0.94 / 1.78 /
       // 3.83 / 9.4 with 32; with 32 free leading bases 2.15 both) while four blocks of
