@@ -309,12 +309,14 @@ bool shape_usable(int s, uint32_t max_band, uint32_t max_q, const SwParams& sp) 
 // in us on both sides (at 300 bp, and 1,000 where it fits, they cross at the same counts):
 //   band 17, 2 x 9 / 4 x 5 words: 12,000 items 192 / 172, 16,000 203 / 206, 24,000 247 / 312,
 //     100,000 796 / 1037; 1 x 34 / 4 x 5 (bands 18 and 19): 30,000 391 / 362, 100,000 987 / 1037
-//   band 50, 32 x 2 / 8 x 9: 1,700 items 101 / 120, 2,200 122 / 119, 3,400 162 / 146, 100,000
+//   band 50, 32 x 2 / 8 x 9: 1,700 items 101 / 120, 2,800 144 / 144, 3,400 162 / 146, 100,000
 //     3905 / 2085
-//   band 50 and 64, 8 x 9 / 2 x 34: 30,000 items 660 / 780, 40,000 891 / 931, 50,000 1075 /
-//     1055, 100,000 2085 / 1926
+//   band 50 and 64, 8 x 9 / 2 x 34: 30,000 items 660 / 780, 50,000 1075 / 1055, 100,000 2085 /
+//     1926; beside a class of as many items on 1 x 34, 21,000 each: 1562 / 1278 a call, 15,000
+//     1303 / 1240
 //   band 64, 8 x 9 / 16 x 9: 1,200 items 118 / 133
-//   band 100, 16 x 9 / 4 x 34: 6,000 items 311 / 326, 7,500 380 / 338, 9,000 412 / 344
+//   band 100, 16 x 9 / 4 x 34: 6,000 items 311 / 326, 9,000 412 / 344 at 3 % of errors; band
+//     128 of 171-344 bases at 5-12 %, whose bands move more, 9,500 items 1027 / 1118 a call
 // Batches no pick fits take any packed shape that does, else the int32 shape of the
 // one-launch path.
 int default_shape(uint32_t max_band, uint32_t max_q, const SwParams& sp, uint32_t items) {
@@ -326,8 +328,8 @@ int default_shape(uint32_t max_band, uint32_t max_q, const SwParams& sp, uint32_
       {23, 20000}, {7, 18000},                        // 34 cells on 1 lane, 36 on 2
       {22, 60000}, {8, 8000},                         // 68 on 1, 40 on 4
       {22, 20000}, {9, 8000},  {10, 1200},            // 68 on 1, 72 on 4, 80 on 8
-      {19, 50000}, {11, 2000}, {24, 0},   {11, 1200},  // 136 on 2, 144 on 8, 128 on 32
-      {20, 7000},  {12, 1200},                        // 272 on 4, 288 on 16
+      {19, 20000}, {11, 3000}, {24, 0},   {11, 1200},  // 136 on 2, 144 on 8, 128 on 32
+      {20, 10000}, {12, 1200},                        // 272 on 4, 288 on 16
       {25, 0},     {13, 0},                           // 320 and 576 on 32
   };
   for (const Pick& p : kPicks)
@@ -490,10 +492,12 @@ int pick_shape(const kira_ctx* ctx, uint32_t max_band, uint32_t max_q, const SwP
 }
 
 // Items the composed path's banded-SW stage is expected to run for n pairs (the count is
-// only known on the device): most candidates are rejected or certified -- 5 % of the
-// pairs reach it with 8 candidates per read, 10 % with 4, 25 % under the router's own
-// bounds.
-inline uint32_t expected_sw_items(uint32_t n) { return n / 8; }
+// only known on the device). Most candidates are rejected or certified: 0.35 to 0.6 of the
+// reads reach it, 5 % of the pairs with 8 candidates a read, 11 % with 4, half with one. Both
+// ways off cost: 171,000 pairs of 100 bases with 8,400 items 288 us on 4 x 9 words, 350 on 1 x
+// 34; 309,000 of 150-250 with 42,000 items 1106 and 970; 25,000 with 1,700 items at band 50
+// 197 us on 32 x 2, 239 on 8 x 9.
+inline uint32_t expected_sw_items(uint32_t n) { return n / 12; }
 
 // Trace slots of that stage: a slot a pair, from 2^20 pairs on for every other pair; the
 // items past them go in a second round. (2M pairs of 150 bases: 10.4 GB of slots for 20.7,

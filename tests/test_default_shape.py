@@ -18,7 +18,7 @@ def _pick(band, q, items, scoring=(1, 4, 6, 1)):
 
 BANDS = [1, 8, 16, 17, 18, 33, 35, 36, 39, 40, 48, 50, 63, 64, 67, 68, 71, 72, 100, 128, 135, 136,
          143, 144, 159, 160, 200, 256, 271]
-ITEMS = [1, 50, 1199, 1200, 1999, 2000, 6999, 7000, 8000, 17999, 18000, 20000, 49999, 50000, 60000,
+ITEMS = [1, 50, 1199, 1200, 2999, 3000, 8000, 9999, 10000, 17999, 18000, 19999, 20000, 60000,
          400_000, 4_000_000]
 
 
