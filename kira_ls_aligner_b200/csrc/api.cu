@@ -482,9 +482,8 @@ int build_planes(kira_ctx* ctx, DevPairs& D, uint64_t read_bytes, uint64_t win_b
   return KIRA_OK;
 }
 
-// Launch shape of the banded SW stage: the tuned choice for the band class if it
-// covers the band, else the smallest shape that does.
-// (`items`: the items the stage is expected to run).
+// Launch shape of the banded SW stage: the tuned choice for the band class if it covers the
+// band, else the default for `items` items (as many as the stage is expected to run).
 int pick_shape(const kira_ctx* ctx, uint32_t max_band, uint32_t max_q, const SwParams& sp,
                uint32_t items) {
   const int t = ctx->tuned_shape[band_class(max_band)];
@@ -541,7 +540,6 @@ uint32_t round_items(kira_ctx* ctx, uint32_t items, int shape, uint32_t max_q) {
 int prepare_bsw(kira_ctx* ctx, uint32_t n_pairs, uint32_t items, uint32_t trace_items,
                 const Maxes& mx, int shape, BswLaunch& B) {
   cudaError_t cerr = cudaSuccess;
-  const BswShapeInfo sh = kBswShapes[shape];
   const uint64_t slot = trace_slot_bytes(shape, mx.q);
   const uint32_t meta_stride = mx.q + 1;
   const uint32_t slot_cap = mx.q + mx.w + 2;
@@ -550,7 +548,7 @@ int prepare_bsw(kira_ctx* ctx, uint32_t n_pairs, uint32_t items, uint32_t trace_
   KIRA_DBUF(ends, DpEnd, B_ENDS, std::max<uint32_t>(items, 1));
   KIRA_DBUF(slots, uint32_t, B_CIG_SLOTS, (uint64_t)slot_cap * std::max<uint32_t>(items, 1));
   KIRA_DBUF(iop, uint32_t, B_ITEM_OF_PAIR, std::max<uint32_t>(n_pairs, 1));
-  B.tg = shape_trace_geom(sh, trace, meta, slot, meta_stride);
+  B.tg = TraceGeom{trace, meta, slot, meta_stride};
   B.ends = ends;
   B.cig_slots = slots;
   B.slot_cap = slot_cap;
@@ -726,7 +724,6 @@ int verify_pipeline(kira_ctx* ctx, DevPairs D, const Maxes& mx, const kira_verif
   M.count_dev = counters + 0;
   M.k = p.myers_k;
   M.per_pair_k = 1;
-  M.tw = std::max<uint32_t>((mx.w + 31) / 32, 1);
   M.lmax = std::max<uint32_t>((mx.q + 31) / 32, 1);
   M.cascade = 1;
   M.out = out;
@@ -1016,7 +1013,7 @@ int plan_bucketed(kira_ctx* ctx, const kira_pairs& P, const DevPairs& D, const k
     B.sp = sp;
     B.bias = packed_bias(sh, sp);
     B.offset = D.band_offset;
-    B.tg = shape_trace_geom(sh, trace + tbase[c], meta + mbase[c], slot[c], qmax[c] + 1);
+    B.tg = TraceGeom{trace + tbase[c], meta + mbase[c], slot[c], qmax[c] + 1};
     B.ends = ends + base[c];
     B.cells = cells_dev;
     B.cig_slots = slots + (uint64_t)base[c] * cap;
@@ -1574,8 +1571,7 @@ cudaError_t run_as_graph(kira_ctx* ctx, const DevPairs& D, const BucketRun& R,
     if (!R.cnt[c]) continue;
     const BswLaunch& B = R.L[c];
     put(B.list), put(B.count), put(B.sp), put(B.offset), put(B.bias), put(B.max_q);
-    put(B.tg.trace), put(B.tg.meta), put(B.tg.slot_bytes), put(B.tg.row_stride);
-    put(B.tg.lane_bytes), put(B.tg.k_cells), put(B.tg.meta_stride), put(B.tg.half);
+    put(B.tg.trace), put(B.tg.meta), put(B.tg.slot_bytes), put(B.tg.meta_stride);
     put(B.ends), put(B.cells), put(B.cig_slots), put(B.slot_cap), put(B.out), put(B.ncig);
     put(B.item_of_pair), put(B.flags), put(B.work), put(B.item_base);
   }
@@ -2833,7 +2829,6 @@ int kira_gpu_myers_batch(kira_ctx* ctx, const kira_pairs* pairs, uint32_t max_k,
   M.count = P.n;
   M.k = (int32_t)max_k;
   M.per_pair_k = 0;
-  M.tw = std::max<uint32_t>((mx.w + 31) / 32, 1);
   M.lmax = std::max<uint32_t>((mx.q + 31) / 32, 1);
   M.dist = dd;
   M.end = de;

@@ -37,18 +37,13 @@ struct SwParams {
   int32_t gof;  // gap_open saturating+ gap_extend (mod.rs:1483)
 };
 
-// Trace arena geometry of one SW launch: item slot s covers
-// trace[s * slot_bytes ...] with row r at r * row_stride; lane g of the group
-// owns bytes [g * lane_bytes, (g + 1) * lane_bytes) of a row, two cells per byte.
+// Trace arena of one SW launch: item slot s covers trace[s * slot_bytes ...], its rows laid
+// out by the shape (BswShape: half a byte a cell; Bsw16Shape: a byte a cell).
 struct TraceGeom {
   uint8_t* trace;
   uint32_t* meta;       // per item: (q_max + 1) words: (row_start << 11) | row_len
   uint64_t slot_bytes;
-  uint32_t row_stride;
-  uint32_t lane_bytes;
-  uint32_t k_cells;     // cells per lane (K); packed shapes: words per lane
   uint32_t meta_stride; // words per item
-  uint32_t half;        // packed shapes: cells per half row (G*K); 0: int32 nibble trace
 };
 
 // Per-item DP result consumed by the traceback kernel.

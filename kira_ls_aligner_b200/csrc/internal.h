@@ -53,7 +53,6 @@ struct MyersLaunch {
   uint32_t count;
   int32_t k;                  // per_pair_k: k < 0 -> router bound per read
   int32_t per_pair_k;
-  uint32_t tw;                // text plane words per pair in shared memory
   uint32_t lmax;              // Peq limbs reserved per lane in shared memory
   int32_t cascade;
   // direct outputs
@@ -183,7 +182,8 @@ struct WfaLaunch {
 // fb_list.
 struct WfaWindow {
   int32_t base, smax, width, lanes;
-  int32_t rows_m, rows_i, rows_d;  // rows of each layer's ring (powers of two)
+  // Rows of each layer's ring: look-back + 1 for M, powers of two for I and D.
+  int32_t rows_m, rows_i, rows_d;
   uint32_t ring_bytes;         // shared bytes of the row rings per pair
   uint32_t pat_bytes;          // shared bytes of the pattern per pair, its guards included
   uint32_t group_bytes;        // shared bytes per pair
@@ -257,11 +257,6 @@ inline uint64_t shape_slot_bytes(const BswShapeInfo& s, uint32_t max_q) {
   const uint64_t r = shape_row_interleave(s);
   const uint64_t rows = ((uint64_t)max_q + 1 + r - 1) / r * r;
   return (rows * shape_row_stride(s) + 15) & ~15ull;
-}
-inline TraceGeom shape_trace_geom(const BswShapeInfo& s, uint8_t* trace, uint32_t* meta,
-                                  uint64_t slot_bytes, uint32_t meta_stride) {
-  return TraceGeom{trace, meta, slot_bytes, shape_row_stride(s), shape_lane_bytes(s),
-                   (uint32_t)s.k, meta_stride, s.packed ? (uint32_t)(s.g * s.k) : 0u};
 }
 
 // Bias of the packed int16 sweep: every biased DP value is >= 0 (F at the far

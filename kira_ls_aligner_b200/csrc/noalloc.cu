@@ -135,7 +135,7 @@ extern "C" int kira_gpu_bsw_batch_noalloc(const kira_pairs* pairs, const kira_sw
   s.gof = c.gap_open + c.gap_extend;
   B.sp = s;
   B.offset = P.band_offset;
-  B.tg = shape_trace_geom(sh, trace, meta, slot, meta_stride);
+  B.tg = TraceGeom{trace, meta, slot, meta_stride};
   B.ends = ends;
   B.cells = nullptr;
   B.cig_slots = slots;
