@@ -100,8 +100,8 @@ struct BswLaunch {
   // bound); trace slots and row metadata are indexed by item - item_lo, every
   // other per-item array by the item itself.
   uint32_t item_lo, item_hi;
-  // 1 / 2: the first / second half of the round's items (their count is on the device),
-  // run on two streams at once; 0: the whole round.
+  // 1 / 2: the first / second half of the first round's items (their count is on the
+  // device), run on two streams at once; 0: the whole round.
   uint32_t split;
   // Packed shapes on batches whose scores pass 255 (the trace keeps H mod 256): items
   // whose walk ended with a value left over (warp_walk_h) are listed here as item_base

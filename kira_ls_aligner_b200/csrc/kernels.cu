@@ -472,16 +472,17 @@ __global__ void __launch_bounds__(128) myers_kernel(DevPairs P, MyersLaunch M) {
 // Banded SW: DP sweep (group of G lanes per item) and traceback (thread per item)
 // ---------------------------------------------------------------------------
 // The items [lo, end) of a launch: its trace round, or with B.split one of the two
-// halves of the round's (device-side) items that run on two streams at once.
+// halves of the first round's (device-side) items that run on two streams at once.
 __device__ __forceinline__ void bsw_range(const BswLaunch& B, uint32_t& lo, uint32_t& end) {
   const uint32_t count = B.count_dev ? *B.count_dev : B.count;
-  lo = B.item_lo;
-  end = max(B.item_hi ? min(count, B.item_hi) : count, lo);
   if (B.split) {
-    const uint32_t mid = lo + (end - lo + 1u) / 2u;
-    if (B.split == 1u) end = mid;
-    else lo = mid;
+    const uint32_t all = B.item_hi ? min(count, B.item_hi) : count, mid = (all + 1u) / 2u;
+    lo = B.split == 1u ? 0u : mid;
+    end = B.split == 1u ? mid : all;
+    return;
   }
+  lo = B.item_lo;
+  end = B.item_hi ? min(count, B.item_hi) : count;
 }
 
 template <int G, int K, int T, int MINB, bool FULL>
