@@ -283,8 +283,9 @@ inline bool packed_trace_wraps(uint32_t max_q, const SwParams& sp) {
 // loses at most a match), so the diagonal is taken wrongly when mismatch is a multiple of
 // 256 plus something of [-match, 2 gof]: 100,000 pairs of 150 bp at match 9, mismatch 247,
 // gaps 0 and 3 lost nearly all their walks and took 4.4 s, on int32 lanes 4.9 ms. What
-// remains is left to the rescue: a jump at the band's edge, or a gap cell 256 below what the gap needs (1 in 100 to
-// 1 in 6,000 short noisy reads on scorings of 10 to 30 a match, none on the default's).
+// remains is left to the rescue: a jump at the band's edge, or a gap cell 256 below what
+// the gap needs (1 in 100 to 1 in 6,000 short noisy reads on scorings of 10 to 30 a match,
+// none on the default's).
 inline bool packed_trace_aliases(const SwParams& sp) {
   const int64_t step = (int64_t)sp.match + sp.mismatch;
   return step > 255 && step % 256 <= sp.match + 2ll * sp.gof;
