@@ -2221,20 +2221,19 @@ int kira_gpu_wfa_batch(kira_ctx* ctx, const kira_pairs* pairs, const kira_wfa_pa
   L.slot_cap = (uint32_t)(2 * (S / min_cost) + 2);
   L.max_score_pp = nullptr;
   L.tbf_pp = nullptr;
-  // Fixed-window passes: 64 diagonals per pair, then 128 for what 64 leave open, placed so
-  // every cell of the highest score stays inside for this batch's leading free text; pairs
-  // still open after that fall back to the general kernel with a warp per pair (their
-  // fronts are the wide ones). A pass that leaves most pairs open is work for nothing, so
-  // one whose scores end before 32, or before mismatches on a 32nd of the longest read, is
-  // left out: the 64 from about 300 bases on with the usual costs, and without a traceback
-  // the 128 too from about 600 on (20,000 reads of 400 bases, 1 / 4 % of errors at most:
-  // 0.49 / 1.67 ms with both, 0.44 / 1.49 with 128 alone; 6,000 of 1,000, no traceback: 0.90
-  // / 3.11 with both, 0.64 / 2.64 with the general kernel alone; free leading text makes
-  // that one's fronts wide from the start: 20,000 of 400 with 40 free, 1.8 against 3.3).
-  // A batch that does not fill the GPU waits for each pass in turn: below 2^15 pairs the 64
-  // go first only where their scores reach mismatches on a 12th of the longest read (24,000
-  // reads of 180-200 bases at 4 %: 1.55 ms with both, 1.48 with 128 alone; 1,000 of them
-  // 1.15 and 1.10).
+  // Fixed-window passes: 64 diagonals per pair, then a wider one for what 64 leave open,
+  // placed so every cell of the highest score stays inside for this batch's leading free
+  // text; pairs still open after that fall back to the general kernel with a warp per pair.
+  // A pass that leaves most pairs open is work for nothing, so one whose scores end before
+  // 32, or before mismatches on a 32nd of the longest read, is left out: the 64 from about
+  // 300 bases on with the usual costs (20,000 reads of 400 bases at 4 %: 1.67 ms with 64 and
+  // 128, 1.49 with 128 alone), and without a traceback the wide one too from about 600 on,
+  // where 128 would end (6,000 of 1,000 at 4 %: 3.5 ms with it, 2.8 with the general kernel
+  // alone; free leading text makes that one's fronts wide from the start: 20,000 of 400 with
+  // 40 free, 1.8 against 3.3). A batch that does not fill the GPU waits for each pass in
+  // turn: below 2^15 pairs the 64 go first only where their scores reach mismatches on a
+  // 12th of the longest read (1,000 reads of 180-200 bases at 4 %: 1.15 ms with both, 1.10
+  // with 128 alone).
   // ctx->wfa_lanes != 0 forces the general kernel alone.
   auto place = [&](int width, int* base) {
     int best = -1;
@@ -2282,8 +2281,26 @@ int kira_gpu_wfa_batch(kira_ctx* ctx, const kira_pairs* pairs, const kira_wfa_pa
       if (add_window(64, b64, s64, 16) > (56u << 10)) add_window(64, b64, s64, 32);
       ++wins;
     }
-    if (s128 >= 16 && serves(s128) && (wins ? S > win[0].smax && s128 > s64 : s128 > s64)) {
-      add_window(128, b128, s128, 32);
+    // The wide pass: 256 diagonals, or as many more as reach mismatches on a 12th of the
+    // longest read, but no more than the batch's scores need. A row takes the diagonals its
+    // score reaches however wide the window is, and a pair left open starts again from its
+    // first row, so the hardest pair's second search was most of a small batch's time.
+    // Measured, 128 / 256 / 384 diagonals: 5,000 pairs of 163-213 bases at 4 % 560 / 276 / 278
+    // us, 30,000 of them 1025 / 718 / 810 (less memory, more warps), 16,000 of 187 without a
+    // traceback 618 / 380 / 401; 1,000 of 700 bases 1774 / 1960 / 662, and of 1,000 2790 /
+    // 2994 / 3200, 1008 with 512. Three blocks of such pairs fit an SM, four where more pairs
+    // wait than are resident (16,000 of 1,000: 384 diagonals 6470, 512 6625; with errors of
+    // 0.5 % at most, which 128 finish, 128 / 384 / 512 693 / 785 / 829).
+    const uint32_t most = n < (1u << 13) ? 72u << 10 : 56u << 10;
+    const int64_t need = (int64_t)L.x * m_max / 12;
+    int width = 128, base = b128, sw = s128;
+    for (int w = 160, b = 0; s128 >= 0 && sw < S && (width < 256 || sw < need); w += 32) {
+      const int sm = place(w, &b);
+      if (add_window(w, b, sm, 32) > most) break;
+      width = w, base = b, sw = sm;
+    }
+    if (sw >= 16 && serves(s128) && (wins ? S > win[0].smax && sw > s64 : sw > s64)) {
+      add_window(width, base, sw, 32);
       ++wins;
     } else if (!wins && s64 >= 16 && serves(s64)) {
       add_window(64, b64, s64, 32);
@@ -2334,7 +2351,19 @@ int kira_gpu_wfa_batch(kira_ctx* ctx, const kira_pairs* pairs, const kira_wfa_pa
   uint64_t blocks = std::min<uint64_t>((csz + gpb - 1) / gpb, (uint64_t)ctx->sms * per_sm);
   blocks = std::min<uint64_t>(blocks,
                               std::max<uint64_t>(1, kWfaScratchBudget / (gpb * group_bytes)));
-  KIRA_DBUF(scratch, uint8_t, B_WFA_SCRATCH, blocks * gpb * group_bytes);
+  // After window passes: a warp per pair, up to 4 warps (pairs) per block, no more than are
+  // resident, and nothing where the last pass reaches every score.
+  const bool general = !wins || S > win[wins - 1].smax;
+  uint64_t groups = blocks * gpb;
+  uint32_t fwpb = 4;
+  if (wins) {
+    while (fwpb > 1 && (uint64_t)fwpb * L.smem_group > (160u << 10)) fwpb >>= 1;
+    int fper = 0;
+    KIRA_CUDA(wfa_blocks_per_sm(32, tb, (size_t)fwpb * L.smem_group, (int)(32 * fwpb), &fper));
+    if (fper < 1) return fail(ctx, KIRA_ERR_INVALID, "WFA fallback: %u shared bytes", L.smem_group);
+    groups = std::min<uint64_t>(groups, (uint64_t)ctx->sms * fper * fwpb);
+  }
+  KIRA_DBUF(scratch, uint8_t, B_WFA_SCRATCH, general ? groups * group_bytes : 1);
   KIRA_DBUF(dout, kira_wfa_result, B_WFA_OUT, n);
   // Flags, then per chunk the fetch counter of the general kernel and the fetch and the
   // fallbacks of each window pass.
@@ -2343,7 +2372,6 @@ int kira_gpu_wfa_batch(kira_ctx* ctx, const kira_pairs* pairs, const kira_wfa_pa
   L.scratch = scratch;
   L.flags = work;
   uint64_t wblocks[2] = {0, 0};
-  uint32_t fwpb = 4;
   for (int i = 0; i < wins; ++i) {
     WfaWindow& X = win[i];
     const uint64_t wpairs = wfa_window_pairs(X);
@@ -2365,12 +2393,6 @@ int kira_gpu_wfa_batch(kira_ctx* ctx, const kira_pairs* pairs, const kira_wfa_pa
   if (wins) {
     KIRA_DBUF(fbl, uint32_t, B_WFA_FB, (uint64_t)wins * n);
     fb = fbl;
-    // Fallback launch shape: 32 lanes per pair, up to 4 warps (pairs) per block; it
-    // uses no more groups than the scratch above holds.
-    while (fwpb > 1 && (uint64_t)fwpb * L.smem_group > (160u << 10)) fwpb >>= 1;
-    int fper = 0;
-    KIRA_CUDA(wfa_blocks_per_sm(32, tb, (size_t)fwpb * L.smem_group, (int)(32 * fwpb), &fper));
-    if (fper < 1) return fail(ctx, KIRA_ERR_INVALID, "WFA fallback: %u shared bytes", L.smem_group);
   }
   uint32_t *ncig = nullptr, *off = nullptr, *sums = nullptr, *ops = nullptr;
   if (tb) {
@@ -2437,13 +2459,13 @@ int kira_gpu_wfa_batch(kira_ctx* ctx, const kira_pairs* pairs, const kira_wfa_pa
         ts = ctx->wfa_tail;
       }
     }
-    if (wins && S > win[wins - 1].smax) {
+    if (wins && general) {
       Lc.list = win[wins - 1].fb_list;
       Lc.list_count = win[wins - 1].fb_count;
       Lc.group = 32;
       KIRA_CUDA(launch_wfa(Dc, Lc,
                            (uint32_t)std::max<uint64_t>(
-                               1, std::min<uint64_t>(blocks * gpb / fwpb, (m + fwpb - 1) / fwpb)),
+                               1, std::min<uint64_t>(groups / fwpb, (m + fwpb - 1) / fwpb)),
                            fwpb, tb, ts));
     } else if (!wins) {
       const uint32_t bl = (uint32_t)std::min<uint64_t>(blocks, (m + gpb - 1) / gpb);
